@@ -390,7 +390,7 @@ int launch_rhs_tc_n(dgtd_op* op, const RhsParams& P) {
   const int64_t end = P.n_elem >= op->n_elem ? op->n_elem_pad : P.n_elem;
   const int64_t tiles = (end - P.e_begin) / C::E;
   const int grid = (int)std::min<int64_t>(tiles, (int64_t)op->ctx->num_sms);
-  kern<<<grid, kTcThreadsAll, C::SMEM, op->stream()>>>(P, T, tiles, op->err.p);
+  kern<<<grid, C::THREADS, C::SMEM, op->stream()>>>(P, T, tiles, op->err.p);
   op->launches++;
   CUDA_TRY(cudaGetLastError());
   return DGTD_OK;
@@ -672,7 +672,8 @@ extern "C" int dgtd_op_create(dgtd_ctx* ctx, const dgtd_op_desc* d, dgtd_op** ou
         }
     };
     // LIFT K is laid out per face, each face padded to KLF = Nfp rounded up to 8,
-    // so the MMAs of a face pair can start while the other pair's flux is formed.
+    // so the MMAs of a face pair can start while the other pair's flux is formed; within a
+    // face the nodes are in the flux units' order (tc_face_node).
     const int KV = dgtd::tc_r8(np), NV = dgtd::tc_nv(N), KLF = dgtd::tc_r8(nfp), KL = 4 * KLF;
     const int NL = dgtd::tc_nl(N);
     std::vector<float> bv, bl;
@@ -686,7 +687,7 @@ extern "C" int dgtd_op_create(dgtd_ctx* ctx, const dgtd_op_desc* d, dgtd_op** ou
     {
       std::vector<float> hl;
       build(NL, KL, [&](int r, int k) -> double {
-        const int f = k / KLF, m = k - f * KLF;
+        const int f = k / KLF, m = dgtd::tc_face_node_of(N, k - f * KLF);
         if (r >= np || m >= nfp) return 0.0;
         return d->lift[r * 4 * nfp + f * nfp + m];
       }, hl);
@@ -2634,7 +2635,7 @@ extern "C" int dgtd_debug_tc_gemm(dgtd_ctx* ctx, const float* a, const float* b,
   return DGTD_OK;
 }
 
-// Point the tensor-core kernel's phase counters (8 x u64, device memory) at
+// Point the tensor-core kernel's phase counters (12 x u64, device memory) at
 // `d_counters`; only builds compiled with -DDGTD_TC_PHASE_TIMERS record them.
 extern "C" int dgtd_debug_set_phase_clock(dgtd_op* op, void* d_counters) {
   if (!op) return set_error(DGTD_ERR_BAD_ARG, "debug_set_phase_clock: null op");

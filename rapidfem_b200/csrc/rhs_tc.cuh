@@ -4,9 +4,11 @@
 //
 // One persistent CTA per SM walks tiles of E elements.  The MMA M dimension is
 // the rows (element, component), split into four lane quarters of QR = M/4
-// rows; quarter q holds elements EQ q .. EQ q + EQ - 1 in rows
-// QR q + 6 (e % EQ) + c, so the six components of an element sit in one warp's
-// TMEM lanes and the curl can be combined with warp shuffles.
+// rows; quarter q holds elements EQ q .. EQ q + EQ - 1, component c of the
+// tile's element e in row QR q + (EQ c + e) mod QR, so the six components of an
+// element sit in one warp's TMEM lanes and the curl can be combined with warp
+// shuffles, and eight neighbouring elements' rows of one component differ
+// mod 8 (conflict-free 16-byte stores of the LIFT operand).
 //   orders 1-4: M = 128, EQ = 5 (E = 20; rows 30, 31 of a quarter are padding),
 //               two TMEM accumulator sets side by side in the columns;
 //   order 5:    M = 64, EQ = 2 (E = 8; rows 12..15 of a quarter are padding).
@@ -24,20 +26,33 @@
 //   LIFT:    C_l[(e,c)][i]     = sum_s Flux[(e,c)][s] * LIFT[i][s]    (rhs.rs:1433-1439)
 //
 // The CTA is warp-specialised so that two tiles are in flight:
-//   flux warps      build tile t's volume operand (tf32 hi/lo of the state,
-//                   written to TMEM by tcgen05.st) and its numerical fluxes
-//                   (rhs.rs:1370-1441) into the LIFT operand in shared memory;
+//   volume warps    build tile t's volume operand (tf32 hi/lo of the state,
+//                   written to TMEM by tcgen05.st);
+//   flux warps      form its numerical fluxes (rhs.rs:1370-1441) into the LIFT
+//                   operand in shared memory;
 //   epilogue warps  finish tile t-1 from its TMEM accumulators: reference
 //                   derivatives -> curl by shuffles, LIFT sum, material scaling
 //                   (rhs.rs:1443-1454) and the mode's update in place (dy, or the
 //                   LSERK4 stage of explicit.rs:122-133 on y and p);
-//   control lane    issues the bulk async loads (state + element records three
-//                   tiles deep, residual register two deep), the MMAs of both
-//                   contractions into one of two TMEM accumulator sets, and the
-//                   bulk async stores.
-// The LIFT operand is formed and multiplied in two halves (faces 0-1, 2-3),
-// each released by its own MMA completion, so the LIFT MMAs of one half run
-// while the flux warps form the other half (or the next tile's volume operand).
+//   control lane    issues the MMAs of both contractions into one of two TMEM
+//                   accumulator sets;
+//   copy lane       issues the bulk async loads (state + element records three
+//                   tiles deep, residual register two deep) and stores.
+// The LIFT operand is formed and multiplied in two halves (faces 0-1, 2-3) by
+// separate warps, each half released by its own MMA completion.
+//
+// What bounds it: the flux warps' chain of one tile (trace loads, fluxes, operand
+// stores) and the epilogue's are both nearly as long as the tile period, with
+// the load/store pipe 60 % busy; HBM and the tensor pipe are not.  One thread per
+// (element, face, four nodes) with 16-byte operand stores, the loads of a face
+// in neighbouring lanes, packed f32x2 arithmetic, a copy lane that refills a
+// slot as soon as it is read and volume warps of their own took five order-4
+// steps of the 48^3 box from 21.7 to 18.1 ms, twenty order-3 steps of the graded
+// 24^3 box from 10.6 to 8.1 ms, ten order-5 steps of 14,586 elements from 2.86
+// to 2.15 ms (one node per thread, 4-byte stores, the flux warps also writing
+// the volume operand, copies issued between the MMAs).  Loading a tile's
+// out-of-tile traces while the previous tile's fluxes are formed measured
+// slower (8, 6 and 4 % more).
 // All hand-offs are mbarriers; every wait is bounded and an expired wait stops
 // the CTA cleanly with an error flag.  The element count is padded on the
 // device to a multiple of E with inert records (PEC faces, zero metric), so
@@ -49,7 +64,10 @@
 #include "tc_util.cuh"
 
 // Phase timers: compiled in only with -DDGTD_TC_PHASE_TIMERS (an instrumented
-// build); otherwise the marks are empty.  One thread per role records.
+// build); otherwise the marks are empty.  One thread per role records the cycles
+// up to each of its marks: volume warps 0 waits, 1 work; flux warps 8 tile wait,
+// 9 trace loads, 2 operand wait, 3 flux; epilogue 10 MMA wait, 4 slot waits,
+// 5 work; control lane 6; copy lane 11 results wait, 7 store read.
 #ifdef DGTD_TC_PHASE_TIMERS
 #define DGTD_TC_MARK(i)                                     \
   do {                                                      \
@@ -68,15 +86,17 @@
 namespace dgtd {
 
 constexpr int kTcTileE = 20;  // elements per tile at orders 1-4 (8 at order 5)
-constexpr int kTcFluxWarps = 12;                          // warps 0..11
-constexpr int kTcEpiWarps = 12;                           // warps 12..23
-constexpr int kTcCtlWarp = kTcFluxWarps + kTcEpiWarps;    // warp 24, lane 0
-constexpr int kTcThreadsAll = (kTcCtlWarp + 1) * 32;
-constexpr int kTcFluxThreads = kTcFluxWarps * 32;
-constexpr int kTcVolGroups = kTcFluxWarps / 4;            // column groups per lane quarter
+// Warps by role: 0..11 epilogue, 12..15 volume operand (both cover whole TMEM
+// lane quarters, quarter = warp % 4), then the order's flux warps, the control
+// and the copy warp.
+constexpr int kTcEpiWarps = 12;
+constexpr int kTcVolWarp = kTcEpiWarps;
+constexpr int kTcVolWarps = 4;
+constexpr int kTcFluxWarp = kTcVolWarp + kTcVolWarps;
 constexpr int kTcEpiGroups = kTcEpiWarps / 4;
+constexpr int kTcMarks = 12;  // phase timers
 constexpr uint32_t kTcWaitLimit = 1u << 19;  // polls per bounded wait (about 2 s)
-static_assert(kTcFluxWarps % 4 == 0 && kTcEpiWarps % 4 == 0, "roles cover whole TMEM lane quarters");
+static_assert(kTcEpiWarps % 4 == 0 && kTcVolWarps == 4, "roles cover whole TMEM lane quarters");
 
 __host__ __device__ constexpr int tc_r8(int x) { return (x + 7) & ~7; }
 __host__ __device__ constexpr int tc_r16(int x) { return (x + 15) & ~15; }
@@ -91,6 +111,21 @@ __host__ __device__ constexpr int tc_tile_e(int n) { return 4 * tc_eq(n); }
 // a 64-row one in steps of 8); the host lays out the constant operands with these.
 __host__ __device__ constexpr int tc_nv(int n) { return tc_m(n) == 64 ? tc_r8(3 * np_of(n)) : tc_r16(3 * np_of(n)); }
 __host__ __device__ constexpr int tc_nl(int n) { return tc_m(n) == 64 ? tc_r8(np_of(n)) : tc_r16(np_of(n)); }
+
+// Face node of LIFT column s of a face (>= Nfp: a padding column).  Four columns
+// are one flux unit, the nodes mg, mg + FG, mg + 2 FG, mg + 3 FG of the face:
+// the FG units of a face are neighbouring lanes, so each of their four loads
+// reads neighbouring nodes, which share 32-byte sectors (four consecutive nodes
+// to a unit: 2.3 times the L1 sector accesses).
+template <int N>
+__host__ __device__ constexpr int tc_face_node(int s) {
+  constexpr int fg = (nfp_of(N) + 3) / 4;
+  return s >= 4 * fg ? nfp_of(N) : fg * (s & 3) + (s >> 2);
+}
+__host__ inline int tc_face_node_of(int order, int s) {
+  return order == 1 ? tc_face_node<1>(s) : order == 2 ? tc_face_node<2>(s) : order == 3 ? tc_face_node<3>(s)
+       : order == 4 ? tc_face_node<4>(s) : tc_face_node<5>(s);
+}
 
 template <int N>
 struct TcCfg {
@@ -121,12 +156,16 @@ struct TcCfg {
   static constexpr int TILE_B = TILE_F * 4;
   static constexpr int META_B = E * kMetaWords * 4;
   // per-thread work
-  static constexpr int SLOTS = E * KL;                                         // flux slots, all faces
-  static constexpr int HSLOTS = SLOTS / 2;                                     // faces 0-1 | faces 2-3
-  static constexpr int ITEMS_H = (HSLOTS + kTcFluxThreads - 1) / kTcFluxThreads;
+  // flux units: (element, face, group of 4 face nodes); faces 0-1 are one half
+  // of the LIFT operand, faces 2-3 the other, each formed by its own warps
+  static constexpr int FG = (NFP + 3) / 4;                                     // node groups per face
+  static constexpr int UNITS_H = E * 2 * FG;                                   // units of a half
+  static constexpr int WARPS_H = (UNITS_H + 31) / 32;                          // flux warps of a half
+  static constexpr int CTL_WARP = kTcFluxWarp + 2 * WARPS_H, COPY_WARP = CTL_WARP + 1;
+  static constexpr int THREADS = (COPY_WARP + 1) * 32;
+  static constexpr bool VEC = NP % 4 == 0;                                     // state rows are whole 16-byte vectors
   static constexpr int KS_H = KL / 16;                                         // LIFT k-steps per half
   static constexpr int VCH = KV / 8;                                           // volume-operand column chunks
-  static constexpr int VCH_PER = (VCH + kTcVolGroups - 1) / kTcVolGroups;
   static constexpr int ECH = (NP + 3) / 4;                                     // epilogue node chunks of 4
   static constexpr int ECH_PER = (ECH + kTcEpiGroups - 1) / kTcEpiGroups;
   // M = 64: a 16-lane TMEM access serves two chunks of 4 columns (one per
@@ -136,7 +175,11 @@ struct TcCfg {
   // byte sizes of the shared-memory operands (hi or lo)
   static constexpr int BV_B = NV * KV * 4;
   static constexpr int BL_B = NL2 * KL * 4;   // stacked hi/lo
-  static constexpr int AL_B = M * KL * 4;
+  // bytes between the 4-column chunks of the LIFT A operand: a warp's flux
+  // stores cover FG chunks of neighbouring elements' rows, and these 16-byte
+  // units of padding spread them over the bank groups
+  static constexpr int AL_CH = M * 16 + 16 * (FG == 4 ? 2 : FG == 2 ? 4 : FG == 1 ? 0 : 3);
+  static constexpr int AL_B = AL_CH * (KL / 4);
   static constexpr int YS_B = tc_r128(TILE_B);
   static constexpr int MS_B = tc_r128(META_B);
   // shared-memory map (bytes)
@@ -149,21 +192,16 @@ struct TcCfg {
   static constexpr int O_M = O_Y + 3 * YS_B;           // 3 element-record slots
   static constexpr int O_P = O_M + 3 * MS_B;           // 2 residual / output slots
   static constexpr int O_TAB = O_P + 2 * YS_B;
-  static constexpr int TAB_B = 4 * NFP + kMaxGather * NFP;
+  // gather tables, each face's list padded to whole 4-node groups
+  static constexpr int TAB_B = kMaxGather * 4 * FG;
   static constexpr int SMEM = O_TAB + tc_r128(TAB_B);
   static_assert(SMEM <= 232448 - 1024, "shared memory per CTA (dynamic + static)");
   static_assert(T_ALO + KV <= TMEM_COLS, "TMEM columns");
   static_assert((TILE_B % 16) == 0 && (META_B % 16) == 0, "bulk copies need 16-byte sizes");
   static_assert(NV <= 256 && NL2 <= 256 && (NV % (M == 128 ? 16 : 8)) == 0 && (NL2 % (M == 128 ? 16 : 8)) == 0,
                 "MMA N limits");
-  // at M = 64 quarter q's rows start at offset q (see tc_row)
-  static_assert((M == 128 || M == 64) && RL <= QR && (!LANE_SETS || (3 + RL <= 16 && ECH % 2 == 0)), "tile shape");
+  static_assert((M == 128 || M == 64) && RL <= QR && (!LANE_SETS || (VEC && ECH % 2 == 0)), "tile shape");
   static_assert(NP <= NL && 3 * NP <= NV, "accumulator columns");
-  // flux slot packing: element (5 bits), face (2), face node (MB), state offset
-  static constexpr int MB = NFP <= 16 ? 4 : 5;
-  static constexpr int OFF_SHIFT = 7 + MB;
-  static_assert(E <= 32 && NFP <= (1 << MB) && TILE_F < (1 << (31 - OFF_SHIFT)), "flux slot packing");
-  static_assert(ITEMS_H <= 2 && VCH_PER <= 4 && ECH_PER <= 8, "per-thread work tables");
   static_assert((KL % 16) == 0, "LIFT halves are whole k-steps");
 };
 
@@ -183,31 +221,44 @@ __device__ __forceinline__ uint32_t tc_set_off(int s) {
   return C::LANE_SETS ? ((uint32_t)(16 * s) << 16) : (uint32_t)(s * C::ACC);
 }
 
-// Row offset of lane quarter q's elements.  At M = 64 the flux warps store the
-// LIFT operand of eight elements at once; starting quarter q's rows at q spreads
-// their rows over more 16-byte bank groups (row mod 8) than a common start.
-template <class C>
-__device__ __forceinline__ int tc_qoff(int q) {
-  return C::LANE_SETS ? q : 0;
-}
-
 // MMA row of (element le, component c) of a tile.
 template <class C>
 __device__ __forceinline__ int tc_row(int le, int c) {
-  return (le / C::EQ) * C::QR + tc_qoff<C>(le / C::EQ) + (le % C::EQ) * 6 + c;
+  return (le / C::EQ) * C::QR + ((C::EQ * c + le) & (C::QR - 1));
 }
 
-// Rotation of a row's node order at M = 64.  The element rows of a state tile
-// are Np = 56 floats apart, so the twelve (element j, component c) rows a warp
-// touches fall into four bank groups of three ((16 j + 24 c) mod 32); the
-// three rows of a group start their four nodes at 0, 1 and 2.
-__device__ __forceinline__ int tc_node_rot(int j, int c) { return j == 0 ? (c >= 4 ? 1 : 0) : (c >= 2 ? 2 : 1); }
+// The (element in quarter, component) of a row r of quarter q: EQ c + el, or a
+// value >= RL for a padding row.
+template <class C>
+__device__ __forceinline__ int tc_row_slot(int q, int r) {
+  return (r - C::EQ * q) & (C::QR - 1);
+}
 
-// a[(v + k) & 3] for a compile-time v and a runtime k in 0..3, without
-// indexing the register array at run time.
-__device__ __forceinline__ float tc_pick4(const float (&a)[4], int v, int k) {
-  const float x0 = a[v & 3], x1 = a[(v + 1) & 3], x2 = a[(v + 2) & 3], x3 = a[(v + 3) & 3];
-  return k == 0 ? x0 : k == 1 ? x1 : k == 2 ? x2 : x3;
+// Nodes i0 .. i0 + 3 of a state row in shared or global memory (one 16-byte access where
+// rows are whole vectors; Np = 10 and 35 go node by node).
+template <class C>
+__device__ __forceinline__ void tc_row_ld(const float* row, int i0, bool on, float (&v)[4]) {
+  if constexpr (C::VEC) {
+    const float4 t = *reinterpret_cast<const float4*>(row + i0);  // a padding lane reads its clamped row
+    v[0] = t.x;
+    v[1] = t.y;
+    v[2] = t.z;
+    v[3] = t.w;
+  } else {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = (on && i0 + u < C::NP) ? row[i0 + u] : 0.f;
+  }
+}
+template <class C>
+__device__ __forceinline__ void tc_row_st(float* row, int i0, bool on, const float (&v)[4]) {
+  if (!on) return;
+  if constexpr (C::VEC) {
+    *reinterpret_cast<float4*>(row + i0) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u < C::NP) row[i0 + u] = v[u];
+  }
 }
 
 // Bounded waits.  A wait gives up after `limit` polls or once another role has
@@ -226,8 +277,8 @@ __device__ __forceinline__ bool tc_wait1(uint64_t* bar, uint32_t parity, volatil
     if (tc::mbar_try_wait(bar, parity)) {
 #ifdef DGTD_TC_PHASE_TIMERS
       const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-      if (l == 0 && (w == 0 || w == kTcFluxWarps || w == kTcCtlWarp))
-        atomicAdd(&g_tc_polls[w == 0 ? 0 : w == kTcFluxWarps ? 1 : 2], (unsigned long long)(i + 1));
+      if (l == 0 && (w == 0 || w == kTcVolWarp || w == kTcFluxWarp))
+        atomicAdd(&g_tc_polls[w == 0 ? 0 : w == kTcVolWarp ? 1 : 2], (unsigned long long)(i + 1));
 #endif
       return true;
     }
@@ -260,16 +311,16 @@ __global__ void k_tc_wait_probe(uint32_t limit, int* err, unsigned long long* wa
 }
 
 template <int N, int MODE>
-__global__ void __launch_bounds__(kTcThreadsAll, 1)
+__global__ void __launch_bounds__(TcCfg<N>::THREADS, 1)
 rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   using C = TcCfg<N>;
   constexpr int NP = C::NP, NFP = C::NFP, E = C::E, M = C::M;
-  constexpr int KV = C::KV, NV = C::NV, KLF = C::KLF, NL = C::NL;
+  constexpr int KV = C::KV, NV = C::NV, KLF = C::KLF, NL = C::NL, FG = C::FG;
   extern __shared__ __align__(1024) unsigned char tsm[];
   __shared__ uint32_t s_tmem;
   __shared__ __align__(8) uint64_t bar_ld[3];   // state + records of a slot landed
-  __shared__ __align__(8) uint64_t bar_p[2];    // residual register of a slot landed
-  __shared__ __align__(8) uint64_t bar_avol;    // flux warps: volume operand in TMEM
+  __shared__ __align__(8) uint64_t bar_p[2];    // residual / output slot ready (residual register landed)
+  __shared__ __align__(8) uint64_t bar_avol;    // volume warps: volume operand in TMEM
   __shared__ __align__(8) uint64_t bar_alift[2];  // flux warps: LIFT operand half (faces 0-1 | 2-3) written
   __shared__ __align__(8) uint64_t bar_l0done;    // the MMAs of LIFT half 0 done (half 0 free)
   __shared__ __align__(8) uint64_t bar_vdone;   // volume MMAs done (TMEM operand free)
@@ -279,17 +330,18 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   volatile int* const abort_flag = &s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool is_flux = warp < kTcFluxWarps;
-  const bool is_epi = !is_flux && warp < kTcCtlWarp;
-  const bool ctl0 = warp == kTcCtlWarp && lane == 0;
+  const bool is_epi = warp < kTcEpiWarps;
+  const bool is_vol = !is_epi && warp < kTcFluxWarp;
+  const bool is_flux = !is_epi && !is_vol && warp < C::CTL_WARP;
+  const bool ctl0 = warp == C::CTL_WARP && lane == 0;
+  const bool copy0 = warp == C::COPY_WARP && lane == 0;
   unsigned char* const alh = tsm + C::O_ALH;
   unsigned char* const all = tsm + C::O_ALL;
   float* const sY0 = reinterpret_cast<float*>(tsm + C::O_Y);
   float* const sM0 = reinterpret_cast<float*>(tsm + C::O_M);
   float* const sP0 = reinterpret_cast<float*>(tsm + C::O_P);
   constexpr int kYStride = C::YS_B / 4, kMStride = C::MS_B / 4;
-  uint8_t* const sFn = tsm + C::O_TAB;
-  uint8_t* const sG = sFn + 4 * NFP;
+  uint8_t* const sG = tsm + C::O_TAB;
   const bool use_p = MODE == kModeLserk && P.read_p;
   const int64_t tile0 = P.e_begin / E;  // the launch covers tiles [tile0, tile0 + n_tiles)
   const int64_t n_my =
@@ -308,9 +360,9 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       tc::mbar_init(&bar_mma[i], 1);
       tc::mbar_init(&bar_epi[i], kTcEpiWarps);
     }
-    tc::mbar_init(&bar_avol, kTcFluxWarps);
-    tc::mbar_init(&bar_alift[0], kTcFluxWarps);
-    tc::mbar_init(&bar_alift[1], kTcFluxWarps);
+    tc::mbar_init(&bar_avol, kTcVolWarps);
+    tc::mbar_init(&bar_alift[0], C::WARPS_H);
+    tc::mbar_init(&bar_alift[1], C::WARPS_H);
     tc::mbar_init(&bar_l0done, 1);
     tc::mbar_init(&bar_vdone, 1);
     tc::mbar_fence_init();
@@ -318,20 +370,22 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   }
   {
     const uint4* src = reinterpret_cast<const uint4*>(T.b_vol);
-    for (int i = tid; i < C::BV_B / 16; i += kTcThreadsAll) {
+    for (int i = tid; i < C::BV_B / 16; i += C::THREADS) {
       reinterpret_cast<uint4*>(tsm + C::O_BVH)[i] = src[i];
       reinterpret_cast<uint4*>(tsm + C::O_BVL)[i] = src[C::BV_B / 16 + i];
     }
     src = reinterpret_cast<const uint4*>(T.b_lift);
-    for (int i = tid; i < C::BL_B / 16; i += kTcThreadsAll) reinterpret_cast<uint4*>(tsm + C::O_BL)[i] = src[i];
-    // LIFT operand padding (rows 30/31 of each quarter, face-padding columns)
+    for (int i = tid; i < C::BL_B / 16; i += C::THREADS) reinterpret_cast<uint4*>(tsm + C::O_BL)[i] = src[i];
+    // LIFT operand padding (the spare rows of each quarter, face-padding columns)
     // must hold finite values and is never written again: start from zero.
-    for (int i = tid; i < C::AL_B / 16; i += kTcThreadsAll) {
+    for (int i = tid; i < C::AL_B / 16; i += C::THREADS) {
       reinterpret_cast<uint4*>(alh)[i] = make_uint4(0, 0, 0, 0);
       reinterpret_cast<uint4*>(all)[i] = make_uint4(0, 0, 0, 0);
     }
-    for (int i = tid; i < 4 * NFP; i += kTcThreadsAll) sFn[i] = T.fnodes[i];
-    for (int i = tid; i < T.n_gather * NFP; i += kTcThreadsAll) sG[i] = T.gtab[i];
+    for (int i = tid; i < T.n_gather * 4 * FG; i += C::THREADS) {
+      const int m = tc_face_node<N>(i % (4 * FG));
+      sG[i] = m < NFP ? T.gtab[(i / (4 * FG)) * NFP + m] : (uint8_t)0;
+    }
   }
   tc::fence_proxy_async_smem();
   tc::tc_fence_before();
@@ -340,98 +394,26 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   const uint32_t tmem = s_tmem;
 
 #ifdef DGTD_TC_PHASE_TIMERS
-  const bool timer_thread = lane == 0 && (warp == 0 || warp == kTcFluxWarps || warp == kTcCtlWarp);
-  unsigned long long clk_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const bool timer_thread = lane == 0 && (warp == 0 || warp == kTcVolWarp || warp == kTcFluxWarp || warp >= C::CTL_WARP);
+  unsigned long long clk_acc[kTcMarks] = {0};
   long long clk_last = clock64();
 #endif
 
-  if (is_flux) {
-    // ================= flux warps: volume operand -> TMEM, fluxes -> LIFT operand
-    const int q4 = warp & 3, vg = warp >> 2;
+  if (is_vol) {
+    // ================= volume warps: tf32 hi/lo of the state -> TMEM
+    const int q4 = warp & 3;
     // the TMEM row this lane writes: its own lane, or (16-lane stores at M = 64)
-    // lane & 15 of the set's lane half, the thread half choosing the columns;
-    // v_row = 6 (element in quarter) + component
-    const int v_row = (C::LANE_SETS ? (lane & 15) : lane) - tc_qoff<C>(q4);
-    const bool lane_real = v_row >= 0 && v_row < C::RL;
-    const int v_src = lane_real ? ((q4 * C::EQ + v_row / 6) * 6 + v_row % 6) * NP : 0;
-    const int v_rot = (C::LANE_SETS && lane_real) ? tc_node_rot(v_row / 6, v_row % 6) : 0;
+    // lane & 15 of the set's lane half, the thread half choosing the columns
+    const int v_slot = tc_row_slot<C>(q4, lane & (C::QR - 1));
+    const bool lane_real = v_slot < C::RL;
+    const int v_src = lane_real ? ((q4 * C::EQ + v_slot % C::EQ) * 6 + v_slot / C::EQ) * NP : 0;
     const uint32_t v_taddr = tmem + ((uint32_t)(q4 * 32) << 16);
-    // flux slots q = (le, face, node-group, node-in-group) of each half (faces
-    // 0-1, then 2-3).  What does not change from tile to tile is packed once:
-    // f_item = le | f << 5 | m << 7 | (offset of the face node's state in the
-    // tile) << (7 + MB), -1 idle; f_off = byte offset of the slot's entry
-    // (component 0) in the LIFT operand.
-    constexpr int kMMask = (1 << C::MB) - 1, kOffShift = C::OFF_SHIFT;
-    int f_item[2][C::ITEMS_H];
-    uint32_t f_off[2][C::ITEMS_H];
-#pragma unroll
-    for (int hh = 0; hh < 2; ++hh)
-#pragma unroll
-      for (int u = 0; u < C::ITEMS_H; ++u) {
-        const int qh = tid + u * kTcFluxThreads;
-        f_item[hh][u] = -1;
-        f_off[hh][u] = 0u;
-        if (qh < C::HSLOTS) {
-          const int q = hh * C::HSLOTS + qh;
-          const int s4 = q & 3, le = (q >> 2) % E, rest = (q >> 2) / E;  // rest = f * (KLF/4) + mg
-          const int f = rest / (KLF / 4), m = (rest % (KLF / 4)) * 4 + s4;
-          if (m < NFP) {
-            f_item[hh][u] = le | (f << 5) | (m << 7) | ((le * 6 * NP + sFn[f * NFP + m]) << kOffShift);
-            const int sl = f * KLF + m;
-            f_off[hh][u] = (uint32_t)((sl >> 2) * (M / 8) * 128 + (sl & 3) * 4 + tc_row<C>(le, 0) * 16);
-          }
-        }
-      }
-    // Out-of-tile neighbour traces of this thread's slots in half hh (global
-    // loads, zero where the neighbour is in the tile or absent).  They are
-    // issued a phase ahead of their use: half 0's before the volume operand is
-    // formed, half 1's right after it (before half 0's fluxes), so their
-    // latency is hidden.
-    // It also leaves, per slot, where the flux finds the neighbour trace:
-    // zi >= 0 its offset in the tile's shared state, -1 the fetched registers,
-    // -2 a PEC face, -3 a port face.
-    const auto nb_fetch = [&](const float* sM, int64_t e0, int hh, float (&nb)[2][6], int (&zi)[2]) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c) nb[u][c] = 0.f;
-        zi[u] = -2;
-        if (u >= C::ITEMS_H || f_item[hh][u] < 0) continue;
-        const int x = f_item[hh][u];
-        const int le = x & 31, f = (x >> 5) & 3, m = (x >> 7) & kMMask;
-        const float* Me = sM + le * kMetaWords;
-        const uint32_t codes = __float_as_uint(Me[41 + (f >> 1)]);
-        const uint32_t code = (f & 1) ? (codes >> 16) : (codes & 0xffffu);
-        const int nbr = __float_as_int(Me[37 + f]);
-        const int kind = (code >> 8) & 3;
-        const int gofs = sG[(code & 0xff) * NFP + m];
-        const int lo = nbr - (int)e0;  // element ids fit in int
-        if (kind == kInterior) {
-          if ((uint32_t)lo < (uint32_t)E) {
-            zi[u] = lo * 6 * NP + gofs;
-          } else {
-            zi[u] = -1;
-            const float* Z = P.y_in + (int64_t)nbr * (6 * NP) + gofs;
-#pragma unroll
-            for (int c = 0; c < 6; ++c) nb[u][c] = __ldg(Z + c * NP);
-          }
-        } else {
-          zi[u] = kind == kPort ? -3 : -2;
-        }
-      }
-    };
     int ys = 0;
     uint32_t ld_par = 0u;  // bit s: parity of the next wait on bar_ld[s]
     for (int64_t it = 0; it < n_my; ++it) {
-      const int64_t tile = tile0 + blockIdx.x + it * gridDim.x;
-      const int64_t e0 = tile * E;
       const float* const sY = sY0 + ys * kYStride;
-      const float* const sM = sM0 + ys * kMStride;
       bool ok = tc_waitw(&bar_ld[ys], (ld_par >> ys) & 1u, abort_flag);
       ld_par ^= 1u << ys;
-      float nb_h[2][2][6];
-      int zi_h[2][2];
-      if (ok) nb_fetch(sM, e0, 0, nb_h[0], zi_h[0]);
       if (ok && it > 0) ok = tc_waitw(&bar_vdone, (uint32_t)((it - 1) & 1), abort_flag);
       if (!ok) {
         *abort_flag = 1;
@@ -442,25 +424,19 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       // ---- volume operand: row (e,c) of this lane, K = nodes, tf32 hi/lo -> TMEM
       if constexpr (C::LANE_SETS) {
         // 8-column unit w: this thread half's 4 columns 8 w + 4 (lane >> 4) ..,
-        // in the lane half of the tile's accumulator set; the four nodes are
-        // read from node v_rot on (no bank replays) and put back in order
+        // in the lane half of the tile's accumulator set
         const uint32_t a_taddr = v_taddr + tc_set_off<C>((int)(it & 1));
 #pragma unroll
-        for (int cc = 0; cc < C::VCH_PER; ++cc) {
-          const int w = vg + kTcVolGroups * cc;
-          if (w < C::VCH) {
-            const int n0 = 8 * w + 4 * (lane >> 4);
-            float v4[4], h[4], l[4];
+        for (int w = 0; w < C::VCH; ++w) {
+          {
+            const float4 v4 = *reinterpret_cast<const float4*>(sY + v_src + 8 * w + 4 * (lane >> 4));
+            const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+            float h[4], l[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              const int k = n0 + ((q + v_rot) & 3);
-              v4[q] = (lane_real && k < NP) ? sY[v_src + k] : 0.f;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const float v = tc_pick4(v4, q, (4 - v_rot) & 3);  // node n0 + q
-              h[q] = tc::tf32_round(v);
-              l[q] = v - h[q];
+              const float x = lane_real ? v[q] : 0.f;
+              h[q] = tc::tf32_round(x);
+              l[q] = x - h[q];
             }
             tc::tmem_st16x2_4(a_taddr + (uint32_t)(C::T_AHI + w * 8), h);
             tc::tmem_st16x2_4(a_taddr + (uint32_t)(C::T_ALO + w * 8), l);
@@ -468,17 +444,28 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
         }
       } else {
 #pragma unroll
-        for (int cc = 0; cc < C::VCH_PER; ++cc) {
-          const int ch = vg + kTcVolGroups * cc;
-          if (ch < C::VCH) {
-            float h[8], l[8];
+        for (int ch = 0; ch < C::VCH; ++ch) {
+          {
+            float x[8], h[8], l[8];
+            if constexpr (C::VEC) {
+#pragma unroll
+              for (int w = 0; w < 2; ++w) {
+                float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (lane_real && ch * 8 + 4 * w < NP) v4 = *reinterpret_cast<const float4*>(sY + v_src + ch * 8 + 4 * w);
+                x[4 * w] = v4.x;
+                x[4 * w + 1] = v4.y;
+                x[4 * w + 2] = v4.z;
+                x[4 * w + 3] = v4.w;
+              }
+            } else {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) x[q] = (lane_real && ch * 8 + q < NP) ? sY[v_src + ch * 8 + q] : 0.f;
+            }
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-              const int k = ch * 8 + q;
-              const float v = (lane_real && k < NP) ? sY[v_src + k] : 0.f;
               // hi/lo split as for the LIFT operand (flux section below)
-              h[q] = tc::tf32_round(v);
-              l[q] = v - h[q];
+              h[q] = tc::tf32_round(x[q]);
+              l[q] = x[q] - h[q];
             }
             tc::tmem_st8(v_taddr + (uint32_t)(C::T_AHI + ch * 8), h);
             tc::tmem_st8(v_taddr + (uint32_t)(C::T_ALO + ch * 8), l);
@@ -490,129 +477,170 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&bar_avol);
       DGTD_TC_MARK(1);
-      // ---- numerical flux (rhs.rs:1370-1441) by halves of the LIFT operand:
-      // faces 0-1, then 2-3.  A half is free once the previous tile's MMAs of
-      // that half are done; its own MMAs then run while the next half is formed.
-      // half 1's traces: before the wait for half 0's operand to be free
-      nb_fetch(sM, e0, 1, nb_h[1], zi_h[1]);
-      // the numerical flux of slot u of half hh (false: an idle slot)
-      const auto flux_of = [&](int hh, int u, float (&fl)[6]) -> bool {
-        if (u >= C::ITEMS_H || f_item[hh][u] < 0) return false;
-        const int x = f_item[hh][u];
-        const int le = x & 31, f = (x >> 5) & 3;
+      ys = ys == 2 ? 0 : ys + 1;
+    }
+  } else if (is_flux) {
+    // ================= flux warps: numerical fluxes -> LIFT operand
+    // This thread's flux unit: node group mg (tc_face_node) of face f of element
+    // le.  One unit per thread and tile: what belongs to the face (normal,
+    // scale, neighbour, face code) is read once for four nodes, and the four
+    // nodes of a row are one 16-byte vector of the LIFT operand.  The lanes of a
+    // face are neighbours, so a load of an out-of-tile trace touches few cache
+    // lines (neighbouring elements in neighbouring lanes: 28.1 against 21.3 ms
+    // for five 48^3 order-4 steps).
+    const int hh = (warp - kTcFluxWarp) / C::WARPS_H;  // half of the LIFT operand
+    const int uh = tid - (kTcFluxWarp + hh * C::WARPS_H) * 32;
+    const bool has_unit = uh < C::UNITS_H;
+    const int mg = uh % FG, le = (uh / FG) % E, f = (2 * hh + uh / (FG * E)) & 3;
+    int own[4];  // offsets of the nodes' states in the tile (component 0)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = tc_face_node<N>(4 * mg + i);
+      own[i] = le * 6 * NP + (has_unit && m < NFP ? (int)T.fnodes[f * NFP + m] : 0);
+    }
+    const uint32_t a_off = (uint32_t)((f * (KLF / 4) + mg) * C::AL_CH + (le / C::EQ) * C::QR * 16);
+    int ys = 0;
+    uint32_t ld_par = 0u;  // bit s: parity of the next wait on bar_ld[s]
+    for (int64_t it = 0; it < n_my; ++it) {
+      const int64_t e0 = (tile0 + blockIdx.x + it * gridDim.x) * E;
+      const float* const sY = sY0 + ys * kYStride;
+      const float* const sM = sM0 + ys * kMStride;
+      bool ok = tc_waitw(&bar_ld[ys], (ld_par >> ys) & 1u, abort_flag);
+      ld_par ^= 1u << ys;
+      DGTD_TC_MARK(8);
+      // The neighbour's traces at the unit's nodes, as pairs of nodes: from the
+      // tile in shared memory when the neighbour is in it, else from L2.
+      float tr[4][6];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) tr[i][c] = 0.f;
+      bool port = false;
+      if (ok && has_unit) {
         const float* Me = sM + le * kMetaWords;
-        const float nx = Me[9 + 3 * f], ny = Me[10 + 3 * f], nz = Me[11 + 3 * f];
-        const float coef = 0.5f * Me[21 + f];
-        const int zi = zi_h[hh][u];
-        const float* Y = sY + (x >> kOffShift);
-        const float ex = Y[0 * NP], ey = Y[1 * NP], ez = Y[2 * NP];
-        const float hx = Y[3 * NP], hy = Y[4 * NP], hz = Y[5 * NP];
-        float jex, jey, jez, jhx, jhy, jhz;
-        float a = P.alpha;
-        if (zi == -3) {
-          // characteristic boundary against a zero incident field (rhs.rs:1380-1386)
-          jex = ex; jey = ey; jez = ez; jhx = hx; jhy = hy; jhz = hz;
-          a = 1.0f;
-        } else if (zi == -2) {
-          // PEC ghost: [E] = 2 E_tan, [H] = 2 H_n (rhs.rs:1387-1402)
-          const float edn = nx * ex + ny * ey + nz * ez;
-          const float hdn = nx * hx + ny * hy + nz * hz;
-          jex = 2.0f * (ex - edn * nx); jey = 2.0f * (ey - edn * ny); jez = 2.0f * (ez - edn * nz);
-          jhx = 2.0f * (hdn * nx); jhy = 2.0f * (hdn * ny); jhz = 2.0f * (hdn * nz);
+        const uint32_t code = reinterpret_cast<const uint16_t*>(Me + 41)[f];
+        const int kind = (int)(code >> 8) & 3;
+        if (kind == kInterior) {
+          const uint32_t g4 = reinterpret_cast<const uint32_t*>(sG)[(code & 0xff) * FG + mg];
+          const int nbr = __float_as_int(Me[37 + f]);
+          const int lo = nbr - (int)e0;  // element ids fit in int
+          const int g0 = g4 & 0xff, g1 = (g4 >> 8) & 0xff, g2 = (g4 >> 16) & 0xff, g3 = g4 >> 24;
+          if ((uint32_t)lo < (uint32_t)E) {
+            const float* Z = sY + lo * 6 * NP;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+              tr[0][c] = Z[g0 + c * NP];
+              tr[1][c] = Z[g1 + c * NP];
+              tr[2][c] = Z[g2 + c * NP];
+              tr[3][c] = Z[g3 + c * NP];
+            }
+          } else {
+            const float* Z = P.y_in + (int64_t)nbr * (6 * NP);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+              tr[0][c] = __ldg(Z + g0 + c * NP);
+              tr[1][c] = __ldg(Z + g1 + c * NP);
+              tr[2][c] = __ldg(Z + g2 + c * NP);
+              tr[3][c] = __ldg(Z + g3 + c * NP);
+            }
+          }
+        } else if (kind == kPec) {
+          // PEC ghost: [E] = 2 E_tan, [H] = 2 H_n (rhs.rs:1387-1402).  Both
+          // products of the flux drop the normal part of a jump, so the ghost
+          // (-E, H) with the jumps 2 E and 0 gives the same flux.
+#pragma unroll
+          for (int c = 0; c < 6; ++c) {
+            const float sg = c < 3 ? -1.f : 1.f;
+            tr[0][c] = sg * sY[own[0] + c * NP];
+            tr[1][c] = sg * sY[own[1] + c * NP];
+            tr[2][c] = sg * sY[own[2] + c * NP];
+            tr[3][c] = sg * sY[own[3] + c * NP];
+          }
         } else {
-          const float (&nb)[6] = nb_h[hh][u];
-          float px = nb[0], py = nb[1], pz = nb[2];
-          float qx = nb[3], qy = nb[4], qz = nb[5];
-          if (zi >= 0) {
-            const float* Z = sY + zi;
-            px = Z[0 * NP]; py = Z[1 * NP]; pz = Z[2 * NP];
-            qx = Z[3 * NP]; qy = Z[4 * NP]; qz = Z[5 * NP];
-          }
-          jex = ex - px; jey = ey - py; jez = ez - pz;
-          jhx = hx - qx; jhy = hy - qy; jhz = hz - qz;
+          port = true;  // characteristic boundary against a zero incident field (rhs.rs:1380-1386)
         }
-        // fe = coef (-n x [H] + a n x (n x [E])), fh = coef (n x [E] + a n x (n x [H]))
-        // (rhs.rs:1420-1432), with n x (n x v) = n (n.v) - v for the unit normal.
-        const float ca = coef * a;
-        const float de = ca * (nx * jex + ny * jey + nz * jez);
-        const float dh = ca * (nx * jhx + ny * jhy + nz * jhz);
-        fl[0] = fmaf(de, nx, fmaf(-ca, jex, -coef * (ny * jhz - nz * jhy)));
-        fl[1] = fmaf(de, ny, fmaf(-ca, jey, -coef * (nz * jhx - nx * jhz)));
-        fl[2] = fmaf(de, nz, fmaf(-ca, jez, -coef * (nx * jhy - ny * jhx)));
-        fl[3] = fmaf(dh, nx, fmaf(-ca, jhx, coef * (ny * jez - nz * jey)));
-        fl[4] = fmaf(dh, ny, fmaf(-ca, jhy, coef * (nz * jex - nx * jez)));
-        fl[5] = fmaf(dh, nz, fmaf(-ca, jhz, coef * (nx * jey - ny * jex)));
-        return true;
-      };
-      // ... into the LIFT operand: hi = tf32(fl), lo = fl - hi (exact,
-      // |lo| <= 2^-11 |fl|).  lo is stored unrounded: the tf32 MMA reads only
-      // its top 19 bits, an error below 2^-10 |lo| <= 2^-21 |fl|, under the
-      // 3xTF32 products' own 2^-22-class terms in the sum of many products.
-      const auto store_of = [&](int hh, int u, const float (&fl)[6]) {
-        const uint32_t off = f_off[hh][u];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-          const float h = tc::tf32_round(fl[c]);
-          *reinterpret_cast<float*>(alh + off + c * 16) = h;
-          *reinterpret_cast<float*>(all + off + c * 16) = fl[c] - h;
-        }
-      };
-      // At M = 64 (one slot per thread and half) both halves' fluxes are formed
-      // before the waits for their operand halves to be free: two independent
-      // chains per thread, and no flux arithmetic behind an MMA completion.
-      float fe[2][6];
-      bool fe_on[2] = {false, false};
-      if constexpr (C::LANE_SETS) {
-        fe_on[0] = flux_of(0, 0, fe[0]);
-        fe_on[1] = flux_of(1, 0, fe[1]);
       }
-      bool half_ok = true;
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        if (it > 0) {
-          const bool free_ok = hh == 0 ? tc_waitw(&bar_l0done, (uint32_t)((it - 1) & 1), abort_flag)
-                                       : tc_waitw(&bar_mma[(it - 1) & 1], (uint32_t)(((it - 1) >> 1) & 1), abort_flag);
-          if (!free_ok) {
-            half_ok = false;
-            break;
-          }
-        }
-        DGTD_TC_MARK(2);
-        if constexpr (C::LANE_SETS) {
-          if (fe_on[hh]) store_of(hh, 0, fe[hh]);
-        } else {
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            float fl[6];
-            if (flux_of(hh, u, fl)) store_of(hh, u, fl);
-          }
-        }
-        tc::fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&bar_alift[hh]);
-      }
-      if (!half_ok) {
+      DGTD_TC_MARK(9);
+      // ---- numerical flux (rhs.rs:1370-1441) into the unit's half of the LIFT
+      // operand, which is free once the previous tile's MMAs of that half are
+      // done; its own MMAs then run while the other half is formed.
+      if (ok && it > 0)
+        ok = hh == 0 ? tc_waitw(&bar_l0done, (uint32_t)((it - 1) & 1), abort_flag)
+                     : tc_waitw(&bar_mma[(it - 1) & 1], (uint32_t)(((it - 1) >> 1) & 1), abort_flag);
+      if (!ok) {
         *abort_flag = 1;
         break;
       }
+      DGTD_TC_MARK(2);
+      if (has_unit) {
+        const float* Me = sM + le * kMetaWords;
+        const float nx = Me[9 + 3 * f], ny = Me[10 + 3 * f], nz = Me[11 + 3 * f];
+        const float coef = -0.5f * Me[21 + f], a = port ? 1.f : P.alpha;
+        // fe = coef (-n x [H] + a n x (n x [E])), fh = coef (n x [E] + a n x (n x [H]))
+        // (rhs.rs:1420-1432), with n x (n x v) = n (n.v) - v for the unit normal,
+        // on the negated jumps j = trace - own and with k = -coef n:
+        // a coef (n (n.[v]) - [v]) = (k.j) (a n) + a coef j.
+        const uint64_t kx = tc::dup2(coef * nx), ky = tc::dup2(coef * ny), kz = tc::dup2(coef * nz);
+        const uint64_t mx = tc::dup2(-coef * nx), my = tc::dup2(-coef * ny), mz = tc::dup2(-coef * nz);
+        const uint64_t ax = tc::dup2(a * nx), ay = tc::dup2(a * ny), az = tc::dup2(a * nz);
+        const uint64_t ca = tc::dup2(-coef * a);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float* Y0 = sY + own[2 * i];
+          const float* Y1 = sY + own[2 * i + 1];
+          const uint64_t ex = tc::sub2(tc::pack2(tr[2 * i][0], tr[2 * i + 1][0]), tc::pack2(Y0[0 * NP], Y1[0 * NP]));
+          const uint64_t ey = tc::sub2(tc::pack2(tr[2 * i][1], tr[2 * i + 1][1]), tc::pack2(Y0[1 * NP], Y1[1 * NP]));
+          const uint64_t ez = tc::sub2(tc::pack2(tr[2 * i][2], tr[2 * i + 1][2]), tc::pack2(Y0[2 * NP], Y1[2 * NP]));
+          const uint64_t hx = tc::sub2(tc::pack2(tr[2 * i][3], tr[2 * i + 1][3]), tc::pack2(Y0[3 * NP], Y1[3 * NP]));
+          const uint64_t hy = tc::sub2(tc::pack2(tr[2 * i][4], tr[2 * i + 1][4]), tc::pack2(Y0[4 * NP], Y1[4 * NP]));
+          const uint64_t hz = tc::sub2(tc::pack2(tr[2 * i][5], tr[2 * i + 1][5]), tc::pack2(Y0[5 * NP], Y1[5 * NP]));
+          const uint64_t de = tc::fma2(kz, ez, tc::fma2(ky, ey, tc::mul2(kx, ex)));
+          const uint64_t dh = tc::fma2(kz, hz, tc::fma2(ky, hy, tc::mul2(kx, hx)));
+          tc::unpack2(tc::fma2(de, ax, tc::fma2(ca, ex, tc::fma2(kz, hy, tc::mul2(my, hz)))), tr[2 * i][0], tr[2 * i + 1][0]);
+          tc::unpack2(tc::fma2(de, ay, tc::fma2(ca, ey, tc::fma2(kx, hz, tc::mul2(mz, hx)))), tr[2 * i][1], tr[2 * i + 1][1]);
+          tc::unpack2(tc::fma2(de, az, tc::fma2(ca, ez, tc::fma2(ky, hx, tc::mul2(mx, hy)))), tr[2 * i][2], tr[2 * i + 1][2]);
+          tc::unpack2(tc::fma2(dh, ax, tc::fma2(ca, hx, tc::fma2(ky, ez, tc::mul2(mz, ey)))), tr[2 * i][3], tr[2 * i + 1][3]);
+          tc::unpack2(tc::fma2(dh, ay, tc::fma2(ca, hy, tc::fma2(kz, ex, tc::mul2(mx, ez)))), tr[2 * i][4], tr[2 * i + 1][4]);
+          tc::unpack2(tc::fma2(dh, az, tc::fma2(ca, hz, tc::fma2(kx, ey, tc::mul2(my, ex)))), tr[2 * i][5], tr[2 * i + 1][5]);
+        }
+        // hi = tf32(flux), lo = flux - hi (exact, |lo| <= 2^-11 |flux|).  lo is
+        // stored unrounded: the tf32 MMA reads only its top 19 bits, an error
+        // below 2^-10 |lo| <= 2^-21 |flux|, under the 3xTF32 products' own
+        // 2^-22-class terms in the sum of many products.
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          const uint32_t off = a_off + (uint32_t)(((C::EQ * c + le) & (C::QR - 1)) * 16);
+          float h[4], l[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            // the operand's padding columns stay zero whatever the fields hold
+            if (tc_face_node<N>(4 * (FG - 1) + i) >= NFP && tc_face_node<N>(4 * mg + i) >= NFP) tr[i][c] = 0.f;
+            h[i] = tc::tf32_round(tr[i][c]);
+            l[i] = tr[i][c] - h[i];
+          }
+          *reinterpret_cast<float4*>(alh + off) = make_float4(h[0], h[1], h[2], h[3]);
+          *reinterpret_cast<float4*>(all + off) = make_float4(l[0], l[1], l[2], l[3]);
+        }
+      }
+      tc::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&bar_alift[hh]);
       DGTD_TC_MARK(3);
       ys = ys == 2 ? 0 : ys + 1;
     }
   } else if (is_epi) {
     // ================= epilogue warps: TMEM -> dy -> mode update, in place
-    const int q4 = warp & 3, eg = (warp - kTcFluxWarps) >> 2;
+    const int q4 = warp & 3, eg = warp >> 2;
     // the TMEM row of this lane: its own lane, or (16-lane loads at M = 64)
-    // lane & 15, the thread half (hb = 0 | 16) reading the second chunk of a
-    // pair; e_row = 6 (element in quarter) + component
-    const int qo = tc_qoff<C>(q4), hb = C::LANE_SETS ? (lane & 16) : 0;
-    const int e_row = (C::LANE_SETS ? (lane & 15) : lane) - qo;
-    const bool lane_real = e_row >= 0 && e_row < C::RL;
-    const int e_le = q4 * C::EQ + (lane_real ? e_row / 6 : C::EQ - 1);
-    const int e_c = lane_real ? e_row % 6 : 5;
+    // lane & 15, the thread half (hb = 0 | 16) reading the second chunk of a pair
+    const int hb = C::LANE_SETS ? (lane & 16) : 0;
+    const int e_slot = tc_row_slot<C>(q4, lane & (C::QR - 1));
+    const bool lane_real = e_slot < C::RL;
+    const int e_el = lane_real ? e_slot % C::EQ : C::EQ - 1, e_c = lane_real ? e_slot / C::EQ : 5;
+    const int e_le = q4 * C::EQ + e_el;
     const int e_fld = e_c / 3, e_t = e_c % 3;
-    const int e_srcA = lane_real ? hb + qo + (e_row / 6) * 6 + 3 * (1 - e_fld) + (e_t + 2) % 3 : lane;
-    const int e_srcB = lane_real ? hb + qo + (e_row / 6) * 6 + 3 * (1 - e_fld) + (e_t + 1) % 3 : lane;
-    const int e_rot = (C::LANE_SETS && lane_real) ? tc_node_rot(e_row / 6, e_c) : 0;
+    const int e_srcA = hb + ((C::EQ * (3 * (1 - e_fld) + (e_t + 2) % 3) + e_le) & (C::QR - 1));
+    const int e_srcB = hb + ((C::EQ * (3 * (1 - e_fld) + (e_t + 1) % 3) + e_le) & (C::QR - 1));
     const float e_sign = e_fld == 0 ? 1.f : -1.f;
     const int e_cA = (e_t + 2) % 3, e_cB = (e_t + 1) % 3;
     const int e_row_off = (e_le * 6 + e_c) * NP;
@@ -633,9 +661,10 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       const int ps = (int)(it & 1);
       const uint32_t ppar = (uint32_t)((it >> 1) & 1);
       bool ok = tc_waitw(&bar_mma[ps], ppar, abort_flag);
+      DGTD_TC_MARK(10);
       if (ok) ok = tc_waitw(&bar_ld[ys], (ld_par >> ys) & 1u, abort_flag);
       ld_par ^= 1u << ys;
-      if (ok && use_p) ok = tc_waitw(&bar_p[ps], ppar, abort_flag);
+      if (ok) ok = tc_waitw(&bar_p[ps], ppar, abort_flag);
       if (!ok) {
         *abort_flag = 1;
         break;
@@ -644,11 +673,10 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       DGTD_TC_MARK(4);
       const float* Me = sM0 + ys * kMStride + e_le * kMetaWords;
       // curl partials (the B one negated) and material scaling with the curl sign folded in
-      const float gA0 = Me[0 * 3 + e_cA], gA1 = Me[1 * 3 + e_cA], gA2 = Me[2 * 3 + e_cA];
-      const float gB0 = -Me[0 * 3 + e_cB], gB1 = -Me[1 * 3 + e_cB], gB2 = -Me[2 * 3 + e_cB];
-      const float inv_w = Me[25 + 3 * e_fld + e_t];
-      const float w_curl = e_sign * inv_w;
-      const float sig_w = Me[31 + 3 * e_fld + e_t];
+      const uint64_t gA0 = tc::dup2(Me[0 * 3 + e_cA]), gA1 = tc::dup2(Me[1 * 3 + e_cA]), gA2 = tc::dup2(Me[2 * 3 + e_cA]);
+      const uint64_t gB0 = tc::dup2(-Me[0 * 3 + e_cB]), gB1 = tc::dup2(-Me[1 * 3 + e_cB]), gB2 = tc::dup2(-Me[2 * 3 + e_cB]);
+      const float inv_wf = Me[25 + 3 * e_fld + e_t];
+      const uint64_t inv_w = tc::dup2(inv_wf), w_curl = tc::dup2(e_sign * inv_wf), sig_w = tc::dup2(-Me[31 + 3 * e_fld + e_t]);
       const float dt_e = P.dt * Me[43];  // the element's own step (batched instances)
       float* const yrow = sY0 + ys * kYStride + e_row_off;
       float* const prow = sP0 + ps * kYStride + e_row_off;  // p in, p out (LSERK) / dy out (Apply)
@@ -682,81 +710,93 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
             tc::tmem_ldw<4>(acc + (uint32_t)(NV + NL + i0), lg);
           }
           tc::tmem_ld_wait();
-          // the mode's update of node i of this row from its dy (yv: y at node i)
-          const auto update = [&](int i, float dy, float yv) {
-            if (MODE == kModeLserk) {
-              // LSERK4 stage (explicit.rs:122-133): p = a p + dt (dy + src); y += b p
-              float k = dy;
-              if (src_here) {
-                if (P.src_vec != nullptr) k = fmaf(P.src_g, __ldg(P.src_vec + g_row + i), k);
-                if (P.src_idx == g_row + i) k += P.src_g;
+          // dy at the four nodes: curl (the shuffles pair this row's partials
+          // with the two other components'), LIFT, materials
+          float dy[4], yv[4];
+          tc_row_ld<C>(yrow, i0, lane_real, yv);
+#pragma unroll
+          for (int u = 0; u < 4; u += 2) {
+            // my contributions: A to curl component (t+1)%3, B to (t+2)%3
+            const uint64_t q0 = tc::pack2(r0[u], r0[u + 1]), q1 = tc::pack2(r1[u], r1[u + 1]), q2 = tc::pack2(r2[u], r2[u + 1]);
+            float A0, A1, B0, B1;
+            tc::unpack2(tc::fma2(gA2, q2, tc::fma2(gA1, q1, tc::mul2(gA0, q0))), A0, A1);
+            tc::unpack2(tc::fma2(gB2, q2, tc::fma2(gB1, q1, tc::mul2(gB0, q0))), B0, B1);
+            const uint64_t sa = tc::pack2(__shfl_sync(0xffffffffu, A0, e_srcA), __shfl_sync(0xffffffffu, A1, e_srcA));
+            const uint64_t sb = tc::pack2(__shfl_sync(0xffffffffu, B0, e_srcB), __shfl_sync(0xffffffffu, B1, e_srcB));
+            const uint64_t li = tc::add2(tc::pack2(lf[u], lf[u + 1]), tc::pack2(lg[u], lg[u + 1]));
+            const uint64_t d = tc::fma2(w_curl, tc::add2(sa, sb),
+                                        tc::fma2(inv_w, li, tc::mul2(sig_w, tc::pack2(yv[u], yv[u + 1]))));
+            tc::unpack2(d, dy[u], dy[u + 1]);
+          }
+          if (MODE == kModeLserk) {
+            // LSERK4 stage (explicit.rs:122-133): p = a p + dt (dy + src); y += b p
+            if (src_here) {
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u;
+                if (lane_real && i < NP) {
+                  if (P.src_vec != nullptr) dy[u] = fmaf(P.src_g, __ldg(P.src_vec + g_row + i), dy[u]);
+                  if (P.src_idx == g_row + i) dy[u] += P.src_g;
+                }
               }
-              float pv = dt_e * k;
-              if (P.read_p) pv = fmaf(P.a, prow[i], pv);
-              prow[i] = pv;
-              yrow[i] = fmaf(P.b, pv, yv);
-            } else if (MODE == kModeKcl) {
-              // KCL stage (explicit_adaptive.rs:84-152) straight to global
-              // memory, in the operation order of the separate stage kernel
-              // (kcl.cuh k_kcl_stage); nothing is staged for the bulk store
-              const int64_t g = g_row + i;
-              float kk = dy;
-              if (src_here) {
-                if (P.src_vec != nullptr) kk += __ldg(P.src_vec + g) * kcl_gs;
-                if (P.src_idx == g) kk += kcl_gs;
+            }
+            float pv[4];
+            const uint64_t dt2 = tc::dup2(dt_e);
+            uint64_t p01 = tc::mul2(dt2, tc::pack2(dy[0], dy[1])), p23 = tc::mul2(dt2, tc::pack2(dy[2], dy[3]));
+            if (P.read_p) {
+              tc_row_ld<C>(prow, i0, lane_real, pv);
+              const uint64_t a2 = tc::dup2(P.a);
+              p01 = tc::fma2(a2, tc::pack2(pv[0], pv[1]), p01);
+              p23 = tc::fma2(a2, tc::pack2(pv[2], pv[3]), p23);
+            }
+            const uint64_t b2 = tc::dup2(P.b);
+            tc::unpack2(p01, pv[0], pv[1]);
+            tc::unpack2(p23, pv[2], pv[3]);
+            tc::unpack2(tc::fma2(b2, p01, tc::pack2(yv[0], yv[1])), yv[0], yv[1]);
+            tc::unpack2(tc::fma2(b2, p23, tc::pack2(yv[2], yv[3])), yv[2], yv[3]);
+            tc_row_st<C>(prow, i0, lane_real, pv);
+            tc_row_st<C>(yrow, i0, lane_real, yv);
+          } else if (MODE == kModeKcl) {
+            // KCL stage (explicit_adaptive.rs:84-152) straight to global
+            // memory, in the operation order of the separate stage kernel
+            // (kcl.cuh k_kcl_stage); nothing is staged for the bulk store
+            const int64_t g = g_row + i0;
+            float ky[4], ke[4], kn[4];
+            tc_row_ld<C>(P.kcl_y + g_row, i0, lane_real, ky);
+            if (P.kcl_stage != 0) tc_row_ld<C>(P.kcl_e + g_row, i0, lane_real, ke);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              float kk = dy[u];
+              if (src_here && lane_real && i0 + u < NP) {
+                if (P.src_vec != nullptr) kk += __ldg(P.src_vec + g + u) * kcl_gs;
+                if (P.src_idx == g + u) kk += kcl_gs;
               }
-              const float f = kcl_h * kk;
-              const float yn = P.kcl_y[g] + P.kcl_b * f;
-              P.kcl_y[g] = yn;
-              P.kcl_e[g] = P.kcl_stage == 0 ? P.kcl_ew * f : P.kcl_e[g] + P.kcl_ew * f;
-              if (P.kcl_next != nullptr) P.kcl_next[g] = yn + P.kcl_amb * f;
-            } else if (MODE == kModeKrylov) {
+              const float fk = kcl_h * kk;
+              ky[u] = ky[u] + P.kcl_b * fk;
+              ke[u] = P.kcl_stage == 0 ? P.kcl_ew * fk : ke[u] + P.kcl_ew * fk;
+              kn[u] = ky[u] + P.kcl_amb * fk;
+            }
+            tc_row_st<C>(P.kcl_y + g_row, i0, lane_real, ky);
+            tc_row_st<C>(P.kcl_e + g_row, i0, lane_real, ke);
+            if (P.kcl_next != nullptr) tc_row_st<C>(P.kcl_next + g_row, i0, lane_real, kn);
+          } else {
+            if (MODE == kModeKrylov) {
               // Krylov matvec of a stored basis vector: its scale and the
               // augmented source coefficient from device memory
-              float w = kry_sig * dy;
+#pragma unroll
+              for (int u = 0; u < 4; ++u) dy[u] *= kry_sig;
               if (src_here) {
-                if (P.src_vec != nullptr) w = fmaf(kry_g, __ldg(P.src_vec + g_row + i), w);
-                if (P.src_idx == g_row + i) w += kry_g;
-              }
-              prow[i] = w;
-            } else {
-              prow[i] = dy;
-            }
-          };
-          if constexpr (C::LANE_SETS) {
-            // curl and LIFT sums node by node (the shuffles pair one node), then
-            // the row's four nodes from node e_rot on (no bank replays on the
-            // state and residual tiles); same arithmetic as below
-            float sc[4], sl[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const float A = fmaf(gA2, r2[u], fmaf(gA1, r1[u], gA0 * r0[u]));
-              const float B = fmaf(gB2, r2[u], fmaf(gB1, r1[u], gB0 * r0[u]));
-              sc[u] = __shfl_sync(0xffffffffu, A, e_srcA) + __shfl_sync(0xffffffffu, B, e_srcB);
-              sl[u] = lf[u] + lg[u];
-            }
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int i = i0 + ((v + e_rot) & 3);
-              if (lane_real && i < NP) {
-                const float yv = yrow[i];
-                update(i, fmaf(w_curl, tc_pick4(sc, v, e_rot), fmaf(inv_w, tc_pick4(sl, v, e_rot), -sig_w * yv)), yv);
+                for (int u = 0; u < 4; ++u) {
+                  const int i = i0 + u;
+                  if (lane_real && i < NP) {
+                    if (P.src_vec != nullptr) dy[u] = fmaf(kry_g, __ldg(P.src_vec + g_row + i), dy[u]);
+                    if (P.src_idx == g_row + i) dy[u] += kry_g;
+                  }
+                }
               }
             }
-          } else {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              // my contributions: A to curl component (t+1)%3, B to (t+2)%3
-              const float A = fmaf(gA2, r2[u], fmaf(gA1, r1[u], gA0 * r0[u]));
-              const float B = fmaf(gB2, r2[u], fmaf(gB1, r1[u], gB0 * r0[u]));
-              const float pa = __shfl_sync(0xffffffffu, A, e_srcA);
-              const float pb = __shfl_sync(0xffffffffu, B, e_srcB);
-              const int i = i0 + u;
-              if (lane_real && i < NP) {
-                const float yv = yrow[i];
-                update(i, fmaf(w_curl, pa + pb, fmaf(inv_w, lf[u] + lg[u], -sig_w * yv)), yv);
-              }
-            }
+            tc_row_st<C>(prow, i0, lane_real, dy);
           }
         }
       }
@@ -768,57 +808,29 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       ys = ys == 2 ? 0 : ys + 1;
     }
   } else if (ctl0) {
-    // ================= control lane: loads, MMAs, stores
-    uint32_t n_ld[3] = {0u, 0u, 0u}, n_p[2] = {0u, 0u}, n_mma[2] = {0u, 0u}, n_vd = 0u, n_l0 = 0u;
+    // ================= control lane: MMAs
+    uint32_t n_mma[2] = {0u, 0u}, n_vd = 0u, n_l0 = 0u;
     const uint32_t idv = tc::idesc_tf32(M, NV), idl = tc::idesc_tf32(M, C::NL2);
-    // Shared-memory descriptors of k-step 0, built once: k-step ks of an R-row
-    // operand adds ks * 2R (16-byte units) to the start-address field, which
-    // cannot carry (shared addresses are below 2^18).  With the k-steps fully
-    // unrolled the issue of an MMA is an add and the instruction itself, so one
-    // thread keeps the tensor pipe fed.
+    // Shared-memory descriptors of k-step 0, built once: a k-step adds two chunks
+    // (in 16-byte units) to the start-address field, which cannot carry (shared
+    // addresses are below 2^18).  With the k-steps fully unrolled the issue of an
+    // MMA is an add and the instruction itself, so one thread keeps the tensor
+    // pipe fed.
     const uint64_t dvh = tc::tf32_step_desc(tc::smem_u32(tsm + C::O_BVH), NV, 0);
     const uint64_t dvl = tc::tf32_step_desc(tc::smem_u32(tsm + C::O_BVL), NV, 0);
     const uint64_t dbl = tc::tf32_step_desc(tc::smem_u32(tsm + C::O_BL), C::NL2, 0);
-    const uint64_t dah = tc::tf32_step_desc(tc::smem_u32(alh), M, 0);
-    const uint64_t dal = tc::tf32_step_desc(tc::smem_u32(all), M, 0);
-    auto load_y = [&](int64_t j) {  // tile j of this CTA -> slot j % 3
-      const int s = (int)(j % 3);
-      const int64_t tile = tile0 + blockIdx.x + j * gridDim.x;
-      tc::mbar_expect_tx(&bar_ld[s], C::TILE_B + C::META_B);
-      tc::bulk_g2s(sY0 + s * kYStride, P.y_in + tile * C::TILE_F, C::TILE_B, &bar_ld[s]);
-      tc::bulk_g2s(sM0 + s * kMStride, P.meta + tile * E * kMetaWords, C::META_B, &bar_ld[s]);
-      ++n_ld[s];
-    };
-    auto load_p = [&](int64_t j) {  // residual register of tile j -> slot j & 1
-      const int s = (int)(j & 1);
-      const int64_t tile = tile0 + blockIdx.x + j * gridDim.x;
-      tc::mbar_expect_tx(&bar_p[s], C::TILE_B);
-      tc::bulk_g2s(sP0 + s * kYStride, P.p + tile * C::TILE_F, C::TILE_B, &bar_p[s]);
-      ++n_p[s];
-    };
-    auto store = [&](int64_t j) {
-      const int64_t gb = (tile0 + (int64_t)blockIdx.x + j * gridDim.x) * C::TILE_F;
-      const float* sy = sY0 + (int)(j % 3) * kYStride;
-      const float* sp = sP0 + (int)(j & 1) * kYStride;
-      if (MODE == kModeApply || MODE == kModeKrylov) {
-        tc::bulk_s2g(P.out + gb, sp, C::TILE_B);
-      } else if (MODE == kModeLserk) {
-        tc::bulk_s2g(P.out + gb, sy, C::TILE_B);
-        if (P.write_p) tc::bulk_s2g(P.p + gb, sp, C::TILE_B);
-      }  // kModeKcl: the epilogue wrote global memory itself
-      tc::bulk_commit();
-    };
-    if (n_my > 0) load_y(0);
-    if (n_my > 1) load_y(1);
-    if (n_my > 0 && use_p) load_p(0);
+    const uint64_t dah = tc::smem_desc(tc::smem_u32(alh), C::AL_CH, 128u);
+    const uint64_t dal = tc::smem_desc(tc::smem_u32(all), C::AL_CH, 128u);
     bool ok = true;
     for (int64_t it = 0; it < n_my && ok; ++it) {
       const int as = (int)(it & 1);
       const uint32_t acc = tmem + tc_set_off<C>(as);
       // the volume A operand: one for both sets (M = 128) or the set's own (M = 64)
       const uint32_t a_base = tmem + (C::LANE_SETS ? tc_set_off<C>(as) : 0u);
-      // volume MMAs: A = state hi/lo (TMEM), B = D hi/lo (shared)
+      // volume MMAs: A = state hi/lo (TMEM), B = D hi/lo (shared); the accumulator
+      // set is free once tile it-2's epilogue is done
       ok = tc_wait1(&bar_avol, (uint32_t)(it & 1), abort_flag);
+      if (ok && it > 1) ok = tc_wait1(&bar_epi[as], (uint32_t)(((it - 2) >> 1) & 1), abort_flag);
       if (!ok) break;
       tc::tc_fence_after();
       DGTD_TC_MARK(6);
@@ -832,16 +844,6 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       }
       tc::mma_commit(&bar_vdone);
       ++n_vd;
-      // Refills: the newest store group is tile it-2's (issued in the previous
-      // iteration); once it has read its slots, they take tile it+1's state
-      // (slot (it+1) % 3) and tile it's residual (slot it & 1).  Waiting after
-      // the volume MMAs are issued keeps the wait off the tensor pipe's path.
-      if (it > 0) {
-        tc::bulk_wait_read0();
-        DGTD_TC_MARK(7);
-        if (it + 1 < n_my) load_y(it + 1);
-        if (use_p) load_p(it);
-      }
       // LIFT MMAs by halves: A = flux hi/lo (shared), B = stacked LIFT hi/lo
       // (shared): columns [NV, NV+NL) collect hi*hi + lo*hi, [NV+NL, NV+2NL)
       // hi*lo + lo*lo.  Half 0's commit frees it for the next tile's flux.
@@ -855,8 +857,8 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
         for (int j = 0; j < C::KS_H; ++j) {
           const int ks = hh * C::KS_H + j;
           const uint64_t bd = dbl + (uint64_t)(2 * C::NL2 * ks);
-          tc::mma_tf32(acc + (uint32_t)NV, dah + (uint64_t)(2 * M * ks), bd, idl, ks > 0 ? 1u : 0u);
-          tc::mma_tf32(acc + (uint32_t)NV, dal + (uint64_t)(2 * M * ks), bd, idl, 1u);
+          tc::mma_tf32(acc + (uint32_t)NV, dah + (uint64_t)(C::AL_CH / 8 * ks), bd, idl, ks > 0 ? 1u : 0u);
+          tc::mma_tf32(acc + (uint32_t)NV, dal + (uint64_t)(C::AL_CH / 8 * ks), bd, idl, 1u);
         }
         if (hh == 0) {
           tc::mma_commit(&bar_l0done);
@@ -866,31 +868,69 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
           ++n_mma[as];
         }
       }
-      if (!ok) break;
-      // results of the previous tile -> HBM
-      if (it > 0) {
-        ok = tc_wait1(&bar_epi[(it - 1) & 1], (uint32_t)(((it - 1) >> 1) & 1), abort_flag);
-        if (!ok) break;
-        DGTD_TC_MARK(6);
-        store(it - 1);
-      }
     }
-    if (ok && n_my > 0) {
-      ok = tc_wait1(&bar_epi[(n_my - 1) & 1], (uint32_t)(((n_my - 1) >> 1) & 1), abort_flag);
-      if (ok) store(n_my - 1);
+    if (!ok) {
+      *abort_flag = 1;
+      // let the MMAs still in flight finish before the CTA exits
+      for (int s = 0; s < 2; ++s)
+        if (n_mma[s]) (void)tc::mbar_wait(&bar_mma[s], (n_mma[s] - 1) & 1u, kTcWaitLimit);
+      if (n_vd) (void)tc::mbar_wait(&bar_vdone, (n_vd - 1) & 1u, kTcWaitLimit);
+      if (n_l0) (void)tc::mbar_wait(&bar_l0done, (n_l0 - 1) & 1u, kTcWaitLimit);
+    }
+  } else if (copy0) {
+    // ================= copy lane: bulk loads and stores.  A tile's slots are
+    // refilled as soon as its results have been read out of them: the state
+    // three tiles on, the residual two.
+    uint32_t n_ld[3] = {0u, 0u, 0u}, n_p[2] = {0u, 0u};
+    auto load_y = [&](int64_t j) {  // tile j of this CTA -> slot j % 3
+      const int s = (int)(j % 3);
+      const int64_t tile = tile0 + blockIdx.x + j * gridDim.x;
+      tc::mbar_expect_tx(&bar_ld[s], C::TILE_B + C::META_B);
+      tc::bulk_g2s(sM0 + s * kMStride, P.meta + tile * E * kMetaWords, C::META_B, &bar_ld[s]);
+      tc::bulk_g2s(sY0 + s * kYStride, P.y_in + tile * C::TILE_F, C::TILE_B, &bar_ld[s]);
+      ++n_ld[s];
+    };
+    auto load_p = [&](int64_t j) {  // slot j & 1: free for tile j's results, with its residual register
+      const int s = (int)(j & 1);
+      if (use_p) {
+        const int64_t tile = tile0 + blockIdx.x + j * gridDim.x;
+        tc::mbar_expect_tx(&bar_p[s], C::TILE_B);
+        tc::bulk_g2s(sP0 + s * kYStride, P.p + tile * C::TILE_F, C::TILE_B, &bar_p[s]);
+      } else {
+        tc::mbar_arrive(&bar_p[s]);
+      }
+      ++n_p[s];
+    };
+    for (int64_t j = 0; j < 3 && j < n_my; ++j) load_y(j);
+    for (int64_t j = 0; j < 2 && j < n_my; ++j) load_p(j);
+    bool ok = true;
+    for (int64_t j = 0; j < n_my; ++j) {
+      ok = tc_wait1(&bar_epi[j & 1], (uint32_t)((j >> 1) & 1), abort_flag);
+      if (!ok) break;
+      DGTD_TC_MARK(11);
+      const int64_t gb = (tile0 + (int64_t)blockIdx.x + j * gridDim.x) * C::TILE_F;
+      const float* sy = sY0 + (int)(j % 3) * kYStride;
+      const float* sp = sP0 + (int)(j & 1) * kYStride;
+      if (MODE == kModeApply || MODE == kModeKrylov) {
+        tc::bulk_s2g(P.out + gb, sp, C::TILE_B);
+      } else if (MODE == kModeLserk) {
+        tc::bulk_s2g(P.out + gb, sy, C::TILE_B);
+        if (P.write_p) tc::bulk_s2g(P.p + gb, sp, C::TILE_B);
+      }  // kModeKcl: the epilogue wrote global memory itself
+      tc::bulk_commit();
+      tc::bulk_wait_read0();
+      DGTD_TC_MARK(7);
+      if (j + 3 < n_my) load_y(j + 3);
+      if (j + 2 < n_my) load_p(j + 2);
     }
     tc::bulk_wait0();
     if (!ok) {
       *abort_flag = 1;
-      // let every async operation still in flight finish before the CTA exits
+      // let the copies still in flight finish before the CTA exits
       for (int s = 0; s < 3; ++s)
         if (n_ld[s]) (void)tc::mbar_wait(&bar_ld[s], (n_ld[s] - 1) & 1u, kTcWaitLimit);
-      for (int s = 0; s < 2; ++s) {
+      for (int s = 0; s < 2; ++s)
         if (n_p[s]) (void)tc::mbar_wait(&bar_p[s], (n_p[s] - 1) & 1u, kTcWaitLimit);
-        if (n_mma[s]) (void)tc::mbar_wait(&bar_mma[s], (n_mma[s] - 1) & 1u, kTcWaitLimit);
-      }
-      if (n_vd) (void)tc::mbar_wait(&bar_vdone, (n_vd - 1) & 1u, kTcWaitLimit);
-      if (n_l0) (void)tc::mbar_wait(&bar_l0done, (n_l0 - 1) & 1u, kTcWaitLimit);
     }
   }
 
@@ -899,7 +939,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   if (tid == 0 && s_abort) atomicExch(err, 1);
 #ifdef DGTD_TC_PHASE_TIMERS
   if (timer_thread && P.phase_clk != nullptr)
-    for (int i = 0; i < 8; ++i) atomicAdd(P.phase_clk + i, clk_acc[i]);
+    for (int i = 0; i < kTcMarks; ++i) atomicAdd(P.phase_clk + i, clk_acc[i]);
 #endif
   if (warp == 0) tc::tmem_dealloc(tmem, C::TMEM_COLS);
 }
