@@ -222,6 +222,24 @@ namespace {
 
 using namespace dgtd;
 
+// Launch a kernel that begins with pdl_wait (or reaches it before it touches
+// anything the stream's earlier kernels use): it may be placed while they end.
+template <class... KArgs, class... Args>
+cudaError_t launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                       Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 // ---- layout conversion (AoS y[(e*Np+i)*6+c] <-> SoA y[(e*6+c)*Np+i])
 // Element e occupies the same 6*Np consecutive values in both layouts, so a
 // conversion permutes values inside element blocks: a CTA stages a chunk of
@@ -233,6 +251,7 @@ template <class TI, class TO, int NP, bool TO_SOA>
 __global__ void __launch_bounds__(256) k_relayout(const TI* __restrict__ src, TO* __restrict__ dst, int64_t n_elem) {
   constexpr int PER = 6 * NP, CH = kRelayoutElems * PER;
   __shared__ TI buf[CH];
+  pdl_wait();
   const int64_t n_chunks = (n_elem + kRelayoutElems - 1) / kRelayoutElems;
   for (int64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
     const int64_t base = ch * CH;
@@ -254,9 +273,12 @@ __global__ void __launch_bounds__(256) k_relayout(const TI* __restrict__ src, TO
     }
     __syncthreads();
   }
+  pdl_launch();  // late: a stage kernel placed earlier takes a whole SM from the blocks still to come
 }
 __global__ void k_gather_f32(const float* __restrict__ src, const int64_t* __restrict__ idx,
                              int64_t n, float* __restrict__ out) {
+  pdl_launch();
+  pdl_wait();
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
     out[k] = src[idx[k]];
 }
@@ -266,6 +288,8 @@ __global__ void k_gather_f32(const float* __restrict__ src, const int64_t* __res
 __global__ void __launch_bounds__(256) k_functionals(const float* __restrict__ y, const int64_t* __restrict__ ptr,
                                                      const int64_t* __restrict__ idx, const double* __restrict__ w,
                                                      double* __restrict__ out) {
+  pdl_launch();
+  pdl_wait();
   __shared__ double part[8];
   const int q = blockIdx.x;
   double s = 0.0;
@@ -302,11 +326,11 @@ int relayout(dgtd_op* op, const TI* src, TO* dst) {
   const int64_t chunks = (n_elem + kRelayoutElems - 1) / kRelayoutElems;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(chunks, (int64_t)op->ctx->num_sms * 16));
   switch (op->np) {
-    case np_of(1): k_relayout<TI, TO, np_of(1), TO_SOA><<<grid, 256, 0, op->stream()>>>(src, dst, n_elem); break;
-    case np_of(2): k_relayout<TI, TO, np_of(2), TO_SOA><<<grid, 256, 0, op->stream()>>>(src, dst, n_elem); break;
-    case np_of(3): k_relayout<TI, TO, np_of(3), TO_SOA><<<grid, 256, 0, op->stream()>>>(src, dst, n_elem); break;
-    case np_of(4): k_relayout<TI, TO, np_of(4), TO_SOA><<<grid, 256, 0, op->stream()>>>(src, dst, n_elem); break;
-    case np_of(5): k_relayout<TI, TO, np_of(5), TO_SOA><<<grid, 256, 0, op->stream()>>>(src, dst, n_elem); break;
+    case np_of(1): CUDA_TRY(launch_pdl(k_relayout<TI, TO, np_of(1), TO_SOA>, grid, 256, 0, op->stream(), src, dst, n_elem)); break;
+    case np_of(2): CUDA_TRY(launch_pdl(k_relayout<TI, TO, np_of(2), TO_SOA>, grid, 256, 0, op->stream(), src, dst, n_elem)); break;
+    case np_of(3): CUDA_TRY(launch_pdl(k_relayout<TI, TO, np_of(3), TO_SOA>, grid, 256, 0, op->stream(), src, dst, n_elem)); break;
+    case np_of(4): CUDA_TRY(launch_pdl(k_relayout<TI, TO, np_of(4), TO_SOA>, grid, 256, 0, op->stream(), src, dst, n_elem)); break;
+    case np_of(5): CUDA_TRY(launch_pdl(k_relayout<TI, TO, np_of(5), TO_SOA>, grid, 256, 0, op->stream(), src, dst, n_elem)); break;
     default: return set_error(DGTD_ERR_UNSUPPORTED, "layout conversion: unsupported order");
   }
   op->launches++;
@@ -337,7 +361,7 @@ int launch_rhs_n(dgtd_op* op, const RhsParams& P) {
   OpTables T{op->dT.p, op->liftT.p, op->fnodes.p, op->gtab.p, op->n_gather};
   const int64_t tiles = (P.n_elem - P.e_begin + C::E - 1) / C::E;
   const int grid = (int)std::min<int64_t>(tiles, (int64_t)op->ctx->num_sms * bps);
-  kern<<<grid, C::THREADS, C::SMEM, op->stream()>>>(P, T);
+  CUDA_TRY(launch_pdl(kern, grid, C::THREADS, C::SMEM, op->stream(), P, T));
   op->launches++;
   CUDA_TRY(cudaGetLastError());
   return DGTD_OK;
@@ -357,7 +381,7 @@ int launch_rhs64_n(dgtd_op* op, const RhsParamsT<double>& P) {
   OpTablesT<double> T{op->dT64.p, op->liftT64.p, op->fnodes.p, op->gtab.p, op->n_gather};
   const int64_t tiles = (P.n_elem - P.e_begin + C::E - 1) / C::E;
   const int grid = (int)std::min<int64_t>(tiles, (int64_t)op->ctx->num_sms * bps);
-  kern<<<grid, C::THREADS, C::SMEM, op->stream()>>>(P, T);
+  CUDA_TRY(launch_pdl(kern, grid, C::THREADS, C::SMEM, op->stream(), P, T));
   op->launches++;
   CUDA_TRY(cudaGetLastError());
   return DGTD_OK;
@@ -390,7 +414,7 @@ int launch_rhs_tc_n(dgtd_op* op, const RhsParams& P) {
   const int64_t end = P.n_elem >= op->n_elem ? op->n_elem_pad : P.n_elem;
   const int64_t tiles = (end - P.e_begin) / C::E;
   const int grid = (int)std::min<int64_t>(tiles, (int64_t)op->ctx->num_sms);
-  kern<<<grid, C::THREADS, C::SMEM, op->stream()>>>(P, T, tiles, op->err.p);
+  CUDA_TRY(launch_pdl(kern, grid, C::THREADS, C::SMEM, op->stream(), P, T, tiles, op->err.p));
   op->launches++;
   CUDA_TRY(cudaGetLastError());
   return DGTD_OK;
@@ -1063,8 +1087,8 @@ extern "C" int dgtd_transient_probes(dgtd_op* op, const float* y0, float dt, int
   DGTD_TRY(dgtd_state_upload(op, y0));
   auto record = [&](int64_t row) -> int {
     if (n_probes == 0) return DGTD_OK;
-    k_gather_f32<<<grid_for(n_probes, 256, op->ctx->num_sms), 256, 0, op->stream()>>>(
-        op->y[op->cur].p, d_probe.p, n_probes, d_pv.p + row * n_probes);
+    CUDA_TRY(launch_pdl(k_gather_f32, (unsigned)grid_for(n_probes, 256, op->ctx->num_sms), 256, 0, op->stream(), 
+        op->y[op->cur].p, d_probe.p, n_probes, d_pv.p + row * n_probes));
     op->launches++;
     CUDA_TRY(cudaGetLastError());
     return DGTD_OK;
@@ -1136,8 +1160,8 @@ extern "C" int dgtd_transient_functionals(dgtd_op* op, const float* y0, float dt
   DGTD_TRY(dgtd_state_upload(op, y0));
   auto record = [&](int64_t row) -> int {
     if (n_fun == 0) return DGTD_OK;
-    k_functionals<<<(unsigned)n_fun, 256, 0, op->stream()>>>(op->y[op->cur].p, d_ptr.p, d_idx.p, d_w.p,
-                                                             d_out.p + row * n_fun);
+    CUDA_TRY(launch_pdl(k_functionals, (unsigned)n_fun, 256, 0, op->stream(), op->y[op->cur].p, d_ptr.p, d_idx.p, d_w.p,
+                                                             d_out.p + row * n_fun));
     op->launches++;
     CUDA_TRY(cudaGetLastError());
     return DGTD_OK;
@@ -1202,8 +1226,8 @@ extern "C" int dgtd_record_functionals(dgtd_op* op, int64_t row) {
   if (!op || op->fn_n < 1) return set_error(DGTD_ERR_BAD_ARG, "record_functionals: no functionals set");
   if (row < 0 || row >= op->fn_rows) return set_error(DGTD_ERR_BAD_ARG, "record_functionals: row out of range");
   CUDA_TRY(cudaSetDevice(op->ctx->device));
-  k_functionals<<<(unsigned)op->fn_n, 256, 0, op->stream()>>>(op->y[op->cur].p, op->fn_ptr.p, op->fn_idx.p,
-                                                              op->fn_w.p, op->fn_out.p + row * op->fn_n);
+  CUDA_TRY(launch_pdl(k_functionals, (unsigned)op->fn_n, 256, 0, op->stream(), op->y[op->cur].p, op->fn_ptr.p, op->fn_idx.p,
+                                                              op->fn_w.p, op->fn_out.p + row * op->fn_n));
   op->launches++;
   CUDA_TRY(cudaGetLastError());
   return DGTD_OK;
@@ -1645,14 +1669,14 @@ int kcl_run(dgtd_op* op, float dt, int64_t steps, int drive, int64_t src_dof, co
   const float* sv = drive == DGTD_DRIVE_VECTOR ? op->src_vec.p : nullptr;
   float* y = op->y[op->cur].p;
   auto attempt = [&]() -> int {
-    dgtd::k_kcl_begin<<<ng, nt, 0, s>>>(dc, y, op->kcl_bak.p, n);
+    CUDA_TRY(launch_pdl(dgtd::k_kcl_begin, ng, nt, 0, s, dc, y, op->kcl_bak.p, n));
     DGTD_TRY(kcl_stages(op, dc, y, src_idx, sv, gv));
-    dgtd::k_kcl_err<<<ng, 256, 0, s>>>(dc, op->kcl_bak.p, y, op->kcl_e.p, op->kcl_part.p, n);
-    dgtd::k_kcl_control<<<1, 256, 0, s>>>(dc, op->kcl_part.p, ng, n);
-    dgtd::k_kcl_restore<<<ng, nt, 0, s>>>(dc, y, op->kcl_bak.p, n);
-    if (d_traj) dgtd::k_kcl_record_state<<<ng, nt, 0, s>>>(dc, y, d_traj, n);
+    CUDA_TRY(launch_pdl(dgtd::k_kcl_err, ng, 256, 0, s, dc, op->kcl_bak.p, y, op->kcl_e.p, op->kcl_part.p, n));
+    CUDA_TRY(launch_pdl(dgtd::k_kcl_control, 1, 256, 0, s, dc, op->kcl_part.p, ng, n));
+    CUDA_TRY(launch_pdl(dgtd::k_kcl_restore, ng, nt, 0, s, dc, y, op->kcl_bak.p, n));
+    if (d_traj) CUDA_TRY(launch_pdl(dgtd::k_kcl_record_state, ng, nt, 0, s, dc, y, d_traj, n));
     if (n_fun > 0)
-      dgtd::k_kcl_record_fun<<<(unsigned)n_fun, 256, 0, s>>>(dc, y, d_ptr, d_idx, d_w, d_fun, n_fun);
+      CUDA_TRY(launch_pdl(dgtd::k_kcl_record_fun, (unsigned)n_fun, 256, 0, s, dc, y, d_ptr, d_idx, d_w, d_fun, n_fun));
     op->launches += 5;
     CUDA_TRY(cudaGetLastError());
     return DGTD_OK;
@@ -1840,7 +1864,7 @@ extern "C" int dgtd_transient_kcl_functionals(dgtd_op* op, const float* y0, floa
   }
   DGTD_TRY(dgtd_state_upload(op, y0));
   if (n_fun > 0) {
-    k_functionals<<<(unsigned)n_fun, 256, 0, s>>>(op->y[op->cur].p, d_ptr.p, d_idx.p, d_w.p, d_out.p);
+    CUDA_TRY(launch_pdl(k_functionals, (unsigned)n_fun, 256, 0, s, op->y[op->cur].p, d_ptr.p, d_idx.p, d_w.p, d_out.p));
     CUDA_TRY(cudaGetLastError());
   }
   int st = kcl_run(op, dt, steps, drive, src_dof, g, ctl, nullptr, n_fun, d_ptr.p, d_idx.p, d_w.p, d_out.p, stats);
@@ -1996,10 +2020,10 @@ int krylov_chunk(dgtd_op* op, const B* v, double t, int m, double tol, int P, do
     CUDA_TRY(cudaMemcpyAsync(&st->dim_total, &acc, sizeof(acc), cudaMemcpyHostToDevice, s));
     CUDA_TRY(cudaStreamSynchronize(s));  // acc is on the host stack
   }
-  k_kry_norm_partials<B><<<nb, nt, 0, s>>>(v, n, pa);
+  CUDA_TRY(launch_pdl(k_kry_norm_partials<B>, nb, nt, 0, s, v, n, pa));
   KRY_TRACE("norm_partials", -1);
   DGTD_TRY(psum(pa));
-  k_kry_start<<<1, kExpmThreads, 0, s>>>(st, pa, nb, t, tol, P, op->kpoly.p, delta, m, op->skip.p);
+  CUDA_TRY(launch_pdl(k_kry_start, 1, kExpmThreads, 0, s, st, pa, nb, t, tol, P, op->kpoly.p, delta, m, op->skip.p));
   KRY_TRACE("start", -1);
   op->launches += 2;
   CUDA_TRY(cudaGetLastError());
@@ -2009,36 +2033,36 @@ int krylov_chunk(dgtd_op* op, const B* v, double t, int m, double tol, int P, do
     DGTD_TRY(phalo(vj));
     DGTD_TRY(kry_matvec<B>(op, vj, w, bvec, src_idx, st->mv, op->skip.p));
     KRY_TRACE("matvec", j);
-    k_kry_dots<B><<<nb, nt, 0, s>>>(v, vb, len, n, j + 1, w, pa, op->skip.p);
+    CUDA_TRY(launch_pdl(k_kry_dots<B>, nb, nt, 0, s, v, vb, len, n, j + 1, w, pa, op->skip.p));
     KRY_TRACE("dots", j);
     DGTD_TRY(psum(pa));
     // the sweeps' register-held columns: the smallest of 4, 8, 12 covering j + 1
     if (j < 4) {
-      k_kry_update_dots<B, 4><<<nb, nt, 0, s>>>(st, v, vb, len, n, j, w, pa, nb, pb, op->skip.p);
+      CUDA_TRY(launch_pdl(k_kry_update_dots<B, 4>, nb, nt, 0, s, st, v, vb, len, n, j, w, pa, nb, pb, op->skip.p));
     } else if (j < 8) {
-      k_kry_update_dots<B, 8><<<nb, nt, 0, s>>>(st, v, vb, len, n, j, w, pa, nb, pb, op->skip.p);
+      CUDA_TRY(launch_pdl(k_kry_update_dots<B, 8>, nb, nt, 0, s, st, v, vb, len, n, j, w, pa, nb, pb, op->skip.p));
     } else {
-      k_kry_update_dots<B, kKryCols><<<nb, nt, 0, s>>>(st, v, vb, len, n, j, w, pa, nb, pb, op->skip.p);
+      CUDA_TRY(launch_pdl(k_kry_update_dots<B, kKryCols>, nb, nt, 0, s, st, v, vb, len, n, j, w, pa, nb, pb, op->skip.p));
     }
     KRY_TRACE("update_dots", j);
     DGTD_TRY(psum(pb));
     if (j < 4) {
-      k_kry_update_norm<B, 4><<<nb, nt, 0, s>>>(st, v, vb, len, n, j, w, pb, nb, pa, op->skip.p);
+      CUDA_TRY(launch_pdl(k_kry_update_norm<B, 4>, nb, nt, 0, s, st, v, vb, len, n, j, w, pb, nb, pa, op->skip.p));
     } else if (j < 8) {
-      k_kry_update_norm<B, 8><<<nb, nt, 0, s>>>(st, v, vb, len, n, j, w, pb, nb, pa, op->skip.p);
+      CUDA_TRY(launch_pdl(k_kry_update_norm<B, 8>, nb, nt, 0, s, st, v, vb, len, n, j, w, pb, nb, pa, op->skip.p));
     } else {
-      k_kry_update_norm<B, kKryCols><<<nb, nt, 0, s>>>(st, v, vb, len, n, j, w, pb, nb, pa, op->skip.p);
+      CUDA_TRY(launch_pdl(k_kry_update_norm<B, kKryCols>, nb, nt, 0, s, st, v, vb, len, n, j, w, pb, nb, pa, op->skip.p));
     }
     KRY_TRACE("update_norm", j);
     DGTD_TRY(psum(pa));
-    k_kry_finish_norm<<<1, kExpmThreads, kExpmSmem, s>>>(st, pa, nb, j, op->skip.p);
+    CUDA_TRY(launch_pdl(k_kry_finish_norm, 1, kExpmThreads, kExpmSmem, s, st, pa, nb, j, op->skip.p));
     KRY_TRACE("finish_norm", j);
     op->launches += 4;
     CUDA_TRY(cudaGetLastError());
   }
-  k_kry_finish_coef<<<1, kExpmThreads, kExpmSmem, s>>>(st);
+  CUDA_TRY(launch_pdl(k_kry_finish_coef, 1, kExpmThreads, kExpmSmem, s, st));
   KRY_TRACE("finish_coef", -1);
-  k_kry_lincomb<B><<<nb, nt, 0, s>>>(v, vb, len, n, st, out);
+  CUDA_TRY(launch_pdl(k_kry_lincomb<B>, nb, nt, 0, s, v, vb, len, n, st, out));
   KRY_TRACE("lincomb", -1);
   op->launches += 2;
   CUDA_TRY(cudaGetLastError());

@@ -82,6 +82,8 @@ __device__ inline double kcl_factor(const KclCtl& c, double err_norm, double pre
 
 __global__ void k_kcl_begin(KclCtl* __restrict__ ctl, const float* __restrict__ y, float* __restrict__ ybak,
                             int64_t n) {
+  pdl_launch();
+  pdl_wait();
   const bool run = ctl->status == kKclRunning && ctl->frame < ctl->steps;
   if (run)
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -98,6 +100,8 @@ __global__ void k_kcl_begin(KclCtl* __restrict__ ctl, const float* __restrict__ 
 __global__ void __launch_bounds__(256) k_kcl_err(const KclCtl* __restrict__ ctl, const float* __restrict__ y_old,
                                                  const float* __restrict__ y_new, const float* __restrict__ err,
                                                  double* __restrict__ partials, int64_t n) {
+  pdl_launch();
+  pdl_wait();
   if (ctl->skip) return;
   __shared__ float part[8];
   const float atol = (float)ctl->atol, rtol = (float)ctl->rtol;
@@ -121,6 +125,8 @@ __global__ void __launch_bounds__(256) k_kcl_err(const KclCtl* __restrict__ ctl,
 // gpu/operator.rs:848-887 and the frame bookkeeping.
 __global__ void __launch_bounds__(256) k_kcl_control(KclCtl* __restrict__ ctl, const double* __restrict__ partials,
                                                      int nb, int64_t n) {
+  pdl_launch();
+  pdl_wait();
   if (ctl->skip) return;
   __shared__ double red[256];
   double s = 0.0;
@@ -171,6 +177,8 @@ __global__ void __launch_bounds__(256) k_kcl_control(KclCtl* __restrict__ ctl, c
 
 __global__ void k_kcl_restore(const KclCtl* __restrict__ ctl, float* __restrict__ y, const float* __restrict__ ybak,
                               int64_t n) {
+  pdl_launch();
+  pdl_wait();
   if (ctl->skip || !ctl->restore) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = ybak[i];
@@ -179,6 +187,8 @@ __global__ void k_kcl_restore(const KclCtl* __restrict__ ctl, float* __restrict_
 // Frame record: the SoA state into row `record` of a device trajectory.
 __global__ void k_kcl_record_state(const KclCtl* __restrict__ ctl, const float* __restrict__ y,
                                    float* __restrict__ traj, int64_t n) {
+  pdl_launch();
+  pdl_wait();
   if (ctl->skip || ctl->record < 0) return;
   float* row = traj + (int64_t)ctl->record * n;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -191,6 +201,8 @@ __global__ void __launch_bounds__(256) k_kcl_record_fun(const KclCtl* __restrict
                                                         const int64_t* __restrict__ idx,
                                                         const double* __restrict__ w, double* __restrict__ out,
                                                         int64_t n_fun) {
+  pdl_launch();
+  pdl_wait();
   if (ctl->skip || ctl->record < 0) return;
   __shared__ double part[8];
   const int q = blockIdx.x;

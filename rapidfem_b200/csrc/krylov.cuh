@@ -178,6 +178,8 @@ template <class B>
 __global__ void __launch_bounds__(kKrylovThreads, 2)
 k_kry_dots(const B* __restrict__ v0, const B* __restrict__ vb, int64_t len, int64_t n, int cols,
            const B* __restrict__ w, double* __restrict__ partials, const int* skip) {
+  pdl_launch();
+  pdl_wait();
   if (*skip) return;
   using KV = KryVec<B>;
   using T = typename KV::T;
@@ -249,6 +251,8 @@ __global__ void __launch_bounds__(kKrylovThreads, 2)
 k_kry_update_dots(KrylovDev* st, const B* __restrict__ v0, const B* __restrict__ vb, int64_t len, int64_t n,
                   int j, B* __restrict__ w, const double* __restrict__ partials_in, int nb_in,
                   double* __restrict__ partials_out, const int* skip) {
+  pdl_launch();
+  pdl_wait();
   static_assert(NC <= kKryCols, "columns");
   if (*skip) return;
   using KV = KryVec<B>;
@@ -317,6 +321,8 @@ __global__ void __launch_bounds__(kKrylovThreads, 2)
 k_kry_update_norm(KrylovDev* st, const B* __restrict__ v0, const B* __restrict__ vb, int64_t len, int64_t n,
                   int j, B* __restrict__ w, const double* __restrict__ partials_in, int nb_in,
                   double* __restrict__ partials_out, const int* skip) {
+  pdl_launch();
+  pdl_wait();
   static_assert(NC <= kKryCols, "columns");
   if (*skip) return;
   using KV = KryVec<B>;
@@ -380,6 +386,8 @@ k_kry_update_norm(KrylovDev* st, const B* __restrict__ v0, const B* __restrict__
 template <class B>
 __global__ void __launch_bounds__(kKrylovThreads, 2)
 k_kry_norm_partials(const B* __restrict__ x, int64_t n, double* __restrict__ partials) {
+  pdl_launch();
+  pdl_wait();
   __shared__ double red[kKrylovThreads / 32];
   double acc[1] = {0.0};
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
@@ -396,6 +404,8 @@ template <class B>
 __global__ void __launch_bounds__(kKrylovThreads, 2)
 k_kry_lincomb(const B* __restrict__ v0, const B* __restrict__ vb, int64_t len, int64_t n, const KrylovDev* st,
               B* __restrict__ out) {
+  pdl_launch();
+  pdl_wait();
   using KV = KryVec<B>;
   using T = typename KV::T;
   __shared__ double c[kKryCols];
@@ -525,6 +535,8 @@ constexpr size_t kExpmSmem = 5 * kKrylovMaxDim * kKrylovMaxDim * sizeof(double);
 // sig[0] = 1/beta, s[0] = e_{P-1}/(eta beta).
 __global__ void k_kry_start(KrylovDev* st, const double* partials, int nblocks, double t, double tol, int P,
                             const double* a, double delta, int max_dim, int* skip) {
+  pdl_launch();
+  pdl_wait();
   __shared__ double s_sums[kKryRow];
   if (st->aborted) {  // uniform: an earlier chunk of the step missed its tolerance
     if (threadIdx.x == 0) {
@@ -598,6 +610,8 @@ __global__ void k_kry_start(KrylovDev* st, const double* partials, int nblocks, 
 // hnext*|exp(tH)_{d-1,0}| < tol (propagator.rs:271-301).  Otherwise record
 // H[j+1,j], the scale and augmented part of V_{j+1} and the next matvec's scalars.
 __global__ void k_kry_finish_norm(KrylovDev* st, const double* partials, int nblocks, int j, int* skip) {
+  pdl_launch();
+  pdl_wait();
   if (*skip) return;
   extern __shared__ double sm[];
   __shared__ double s_hnext;
@@ -674,6 +688,8 @@ __global__ void k_kry_finish_norm(KrylovDev* st, const double* partials, int nbl
 
 // End of a chunk: coef_i = beta * exp(tH)_{i,0} * sig_i over the final dim.
 __global__ void k_kry_finish_coef(KrylovDev* st) {
+  pdl_launch();
+  pdl_wait();
   extern __shared__ double sm[];
   __shared__ int s_done;
   const int d = st->dim;

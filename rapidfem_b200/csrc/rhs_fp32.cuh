@@ -86,13 +86,13 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
   uint8_t* sG = sFn + 4 * NFP;
   const int tid = threadIdx.x;
 
-  if (P.skip != nullptr && *P.skip) return;  // uniform: nothing to do for this launch
-
   for (int i = tid; i < 3 * NP * NP; i += blockDim.x) sD[i] = T.dT[i];
   for (int i = tid; i < NF * NP; i += blockDim.x) sL[i] = T.liftT[i];
   for (int i = tid; i < 4 * NFP; i += blockDim.x) sFn[i] = T.fnodes[i];
   for (int i = tid; i < T.n_gather * NFP; i += blockDim.x) sG[i] = T.gtab[i];
 
+  pdl_wait();
+  if (P.skip != nullptr && *P.skip) return;  // uniform: nothing to do for this launch
   R kry_sig = 1, kry_g = 0;
   if (MODE == kModeKrylov) {
     kry_sig = (R)P.kry[0];
@@ -348,6 +348,9 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
       }
     }
   }
+  // Several of these CTAs share an SM: a next launch let in earlier is placed
+  // wherever there is room, unevenly (the f64 kernel: 13 % slower).
+  pdl_launch();
 }
 
 // FP32 engine (stage, RHS and the Krylov matvec of an f32 basis); TD = 2 is

@@ -344,14 +344,10 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   uint8_t* const sG = tsm + C::O_TAB;
   const bool use_p = MODE == kModeLserk && P.read_p;
   const int64_t tile0 = P.e_begin / E;  // the launch covers tiles [tile0, tile0 + n_tiles)
-  const int64_t n_my =
-      n_tiles > (int64_t)blockIdx.x ? (n_tiles - (int64_t)blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
 
-  // a launch flagged off (adaptive stepping past its last attempt) does
-  // nothing; the flag is read before any barrier or TMEM allocation
-  if (P.skip != nullptr && *P.skip) return;
-
-  // ---- set-up: TMEM, barriers, constant operands, tables
+  // ---- set-up: TMEM, barriers, constant operands, tables (while the previous
+  // launch still runs, on SMs that it leaves)
+  pdl_launch();
   if (warp == 0) tc::tmem_alloc(&s_tmem, C::TMEM_COLS);
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) tc::mbar_init(&bar_ld[i], 1);
@@ -392,6 +388,12 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = s_tmem;
+  pdl_wait();
+  // a launch flagged off (adaptive stepping past its last attempt) has no tiles
+  const bool off = P.skip != nullptr && *P.skip;
+  const int64_t n_my = !off && n_tiles > (int64_t)blockIdx.x
+                           ? (n_tiles - (int64_t)blockIdx.x + gridDim.x - 1) / gridDim.x
+                           : 0;
 
 #ifdef DGTD_TC_PHASE_TIMERS
   const bool timer_thread = lane == 0 && (warp == 0 || warp == kTcVolWarp || warp == kTcFluxWarp || warp >= C::CTL_WARP);

@@ -67,3 +67,58 @@ def test_a_nonfinite_element_stays_local(ctx, order):
     far = np.array([q for q in range(m.n_tets) if q not in near])
     assert np.isnan(got[e]).all()
     assert np.array_equal(got[far], clean[far])
+
+
+# ---- stages queued back to back (each kernel is placed while its predecessor
+# ends) against the same stages with the stream drained in between: equal to
+# the bit, or a kernel read its input too early
+
+def _one_by_one(ctx, gop, h, steps, drive=None, g=None):
+    for k in range(steps):
+        for s in range(5):
+            gop.lserk_stage(h, s, drive=drive, g=0.0 if g is None else float(g[k]))
+            ctx.synchronize()
+
+
+@pytest.mark.parametrize("engine", [_native.ENGINE_TF32X3, _native.ENGINE_FP32], ids=["tf32x3", "fp32"])
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("cells,shuffled", [((1, 1, 1), False), ((3, 3, 3), False), ((8, 8, 8), False),
+                                            ((8, 8, 8), True), ((14, 13, 11), False), ((14, 13, 11), True)],
+                         ids=["one_tile", "few_tiles", "8", "8_shuffled", "14", "14_shuffled"])
+def test_a_run_equals_its_stages(ctx, engine, order, cells, shuffled):
+    m = O.structured_box_jittered(*cells, 1.0, 1.0, 1.0, 0.1, 5)
+    if shuffled:
+        m = O.Mesh(m.nodes, np.ascontiguousarray(m.tets[np.random.default_rng(1).permutation(m.n_tets)]))
+    gop = G.GpuOperator(ctx, O.MaxwellOperator(m, order, 1.0))
+    gop.set_engine(engine)
+    n = gop.n_dof()
+    rng = np.random.default_rng(order)
+    y = rng.standard_normal(n).astype(np.float32)
+    h = 0.05 / (max(cells) * order * order)
+    g = rng.standard_normal(18)
+    for steps, drive in ((1, None), (2, ("point", n // 2)), (18, None), (17, ("point", n - 1))):
+        gop.upload(y)
+        gop.run_lserk(h, steps, drive=drive, g=None if drive is None else g[:steps])
+        got = gop.download()
+        gop.upload(y)
+        _one_by_one(ctx, gop, h, steps, drive, None if drive is None else g.astype(np.float32))
+        assert np.array_equal(got, gop.download())
+
+
+def test_runs_on_two_streams(ctx):
+    """Two operators stepping at once on streams of their own."""
+    other = G.GpuContext(0)
+    m = O.structured_box(9, 8, 7)
+    host = O.MaxwellOperator(m, 3, 1.0)
+    ops = [G.GpuOperator(c, host) for c in (ctx, other)]
+    y = np.random.default_rng(3).standard_normal(ops[0].n_dof()).astype(np.float32)
+    for op in ops:
+        op.upload(y)
+    for _ in range(20):
+        for op in ops:
+            op.run_lserk(1e-3, 5)
+    a, b = (op.download() for op in ops)
+    ops[0].upload(y)
+    for _ in range(20):
+        ops[0].run_lserk(1e-3, 5)
+    assert np.array_equal(a, b) and np.array_equal(a, ops[0].download())
