@@ -711,7 +711,7 @@ extern "C" int dgtd_op_create(dgtd_ctx* ctx, const dgtd_op_desc* d, dgtd_op** ou
     {
       std::vector<float> hl;
       build(NL, KL, [&](int r, int k) -> double {
-        const int f = k / KLF, m = dgtd::tc_face_node_of(N, k - f * KLF);
+        const int f = k / KLF, m = dgtd::tc_face_node(N, k - f * KLF);
         if (r >= np || m >= nfp) return 0.0;
         return d->lift[r * 4 * nfp + f * nfp + m];
       }, hl);
@@ -2666,16 +2666,3 @@ extern "C" int dgtd_debug_set_phase_clock(dgtd_op* op, void* d_counters) {
   op->phase_clk = static_cast<unsigned long long*>(d_counters);
   return DGTD_OK;
 }
-
-#ifdef DGTD_TC_PHASE_TIMERS
-// Instrumented builds only: mbarrier polls of the three timed threads.
-extern "C" int dgtd_debug_tc_polls(unsigned long long* host3, int reset) {
-  if (reset) {
-    unsigned long long z[3] = {0, 0, 0};
-    CUDA_TRY(cudaMemcpyToSymbol(dgtd::g_tc_polls, z, sizeof(z)));
-    return DGTD_OK;
-  }
-  CUDA_TRY(cudaMemcpyFromSymbol(host3, dgtd::g_tc_polls, sizeof(unsigned long long) * 3));
-  return DGTD_OK;
-}
-#endif

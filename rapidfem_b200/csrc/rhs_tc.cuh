@@ -86,17 +86,11 @@
 namespace dgtd {
 
 constexpr int kTcTileE = 20;  // elements per tile at orders 1-4 (8 at order 5)
-// Warps by role: 0..11 epilogue, 12..15 volume operand (both cover whole TMEM
-// lane quarters, quarter = warp % 4), then the order's flux warps, the control
-// and the copy warp.
-constexpr int kTcEpiWarps = 12;
-constexpr int kTcVolWarp = kTcEpiWarps;
-constexpr int kTcVolWarps = 4;
-constexpr int kTcFluxWarp = kTcVolWarp + kTcVolWarps;
-constexpr int kTcEpiGroups = kTcEpiWarps / 4;
+// Warps by role: epilogue, 4 volume operand (both cover whole TMEM lane
+// quarters, quarter = warp % 4), then the order's flux warps, the control and
+// the copy warp.
 constexpr int kTcMarks = 12;  // phase timers
 constexpr uint32_t kTcWaitLimit = 1u << 19;  // polls per bounded wait (about 2 s)
-static_assert(kTcEpiWarps % 4 == 0 && kTcVolWarps == 4, "roles cover whole TMEM lane quarters");
 
 __host__ __device__ constexpr int tc_r8(int x) { return (x + 7) & ~7; }
 __host__ __device__ constexpr int tc_r16(int x) { return (x + 15) & ~15; }
@@ -112,19 +106,20 @@ __host__ __device__ constexpr int tc_tile_e(int n) { return 4 * tc_eq(n); }
 __host__ __device__ constexpr int tc_nv(int n) { return tc_m(n) == 64 ? tc_r8(3 * np_of(n)) : tc_r16(3 * np_of(n)); }
 __host__ __device__ constexpr int tc_nl(int n) { return tc_m(n) == 64 ? tc_r8(np_of(n)) : tc_r16(np_of(n)); }
 
-// Face node of LIFT column s of a face (>= Nfp: a padding column).  Four columns
-// are one flux unit, the nodes mg, mg + FG, mg + 2 FG, mg + 3 FG of the face:
-// the FG units of a face are neighbouring lanes, so each of their four loads
+// Face nodes of a flux unit: two where the units then still fit one per thread
+// beside the other roles (the chain of loads, flux and stores per thread is half
+// as long: 82,944 order-3 elements 76.6 -> 70.8 us per stage, 279,936 order-2
+// elements 167 -> 146 us, 14,586 order-5 elements 38.5 -> 37.7 us), four at
+// order 4, where two would take 20 warps.
+__host__ __device__ constexpr int tc_fn(int n) { return n == 4 ? 4 : 2; }
+// Face node of LIFT column s of a face (>= Nfp: a padding column).  FN = 2 or 4
+// consecutive columns are one flux unit, the nodes mg, mg + FG, .. of the face:
+// the FG units of a face are neighbouring lanes, so each of their FN loads
 // reads neighbouring nodes, which share 32-byte sectors (four consecutive nodes
 // to a unit: 2.3 times the L1 sector accesses).
-template <int N>
-__host__ __device__ constexpr int tc_face_node(int s) {
-  constexpr int fg = (nfp_of(N) + 3) / 4;
-  return s >= 4 * fg ? nfp_of(N) : fg * (s & 3) + (s >> 2);
-}
-__host__ inline int tc_face_node_of(int order, int s) {
-  return order == 1 ? tc_face_node<1>(s) : order == 2 ? tc_face_node<2>(s) : order == 3 ? tc_face_node<3>(s)
-       : order == 4 ? tc_face_node<4>(s) : tc_face_node<5>(s);
+__host__ __device__ constexpr int tc_face_node(int n, int s) {
+  const int fn = tc_fn(n), fg = (nfp_of(n) + fn - 1) / fn;
+  return s >= fn * fg ? nfp_of(n) : fg * (s % fn) + s / fn;
 }
 
 template <int N>
@@ -156,29 +151,33 @@ struct TcCfg {
   static constexpr int TILE_B = TILE_F * 4;
   static constexpr int META_B = E * kMetaWords * 4;
   // per-thread work
-  // flux units: (element, face, group of 4 face nodes); faces 0-1 are one half
+  // flux units: (element, face, group of FN face nodes); faces 0-1 are one half
   // of the LIFT operand, faces 2-3 the other, each formed by its own warps
-  static constexpr int FG = (NFP + 3) / 4;                                     // node groups per face
+  static constexpr int FN = tc_fn(N);
+  static constexpr int FG = (NFP + FN - 1) / FN;                                     // node groups per face
   static constexpr int UNITS_H = E * 2 * FG;                                   // units of a half
   static constexpr int WARPS_H = (UNITS_H + 31) / 32;                          // flux warps of a half
-  static constexpr int CTL_WARP = kTcFluxWarp + 2 * WARPS_H, COPY_WARP = CTL_WARP + 1;
+  static constexpr int EPI_WARPS = 12;
+  static constexpr int VOL_WARP = EPI_WARPS, VOL_WARPS = 4, EPI_GROUPS = EPI_WARPS / 4;
+  static constexpr int FLUX_WARP = VOL_WARP + VOL_WARPS;
+  static constexpr int CTL_WARP = FLUX_WARP + 2 * WARPS_H, COPY_WARP = CTL_WARP + 1;
   static constexpr int THREADS = (COPY_WARP + 1) * 32;
   static constexpr bool VEC = NP % 4 == 0;                                     // state rows are whole 16-byte vectors
   static constexpr int KS_H = KL / 16;                                         // LIFT k-steps per half
   static constexpr int VCH = KV / 8;                                           // volume-operand column chunks
   static constexpr int ECH = (NP + 3) / 4;                                     // epilogue node chunks of 4
-  static constexpr int ECH_PER = (ECH + kTcEpiGroups - 1) / kTcEpiGroups;
+  static constexpr int ECH_PER = (ECH + EPI_GROUPS - 1) / EPI_GROUPS;
   // M = 64: a 16-lane TMEM access serves two chunks of 4 columns (one per
   // thread half): the volume operand's K in VCH units of 8, the accumulator's
   // nodes in EPAIRS units of 8
-  static constexpr int EPAIRS = (ECH + 1) / 2, EPAIR_PER = (EPAIRS + kTcEpiGroups - 1) / kTcEpiGroups;
+  static constexpr int EPAIRS = (ECH + 1) / 2, EPAIR_PER = (EPAIRS + EPI_GROUPS - 1) / EPI_GROUPS;
   // byte sizes of the shared-memory operands (hi or lo)
   static constexpr int BV_B = NV * KV * 4;
   static constexpr int BL_B = NL2 * KL * 4;   // stacked hi/lo
   // bytes between the 4-column chunks of the LIFT A operand: a warp's flux
   // stores cover FG chunks of neighbouring elements' rows, and these 16-byte
   // units of padding spread them over the bank groups
-  static constexpr int AL_CH = M * 16 + 16 * (FG == 4 ? 2 : FG == 2 ? 4 : FG == 1 ? 0 : 3);
+  static constexpr int AL_CH = M * 16 + 16 * (N == 4 ? 2 : N == 2 ? 4 : N == 1 ? 0 : 3);
   static constexpr int AL_B = AL_CH * (KL / 4);
   static constexpr int YS_B = tc_r128(TILE_B);
   static constexpr int MS_B = tc_r128(META_B);
@@ -192,8 +191,8 @@ struct TcCfg {
   static constexpr int O_M = O_Y + 3 * YS_B;           // 3 element-record slots
   static constexpr int O_P = O_M + 3 * MS_B;           // 2 residual / output slots
   static constexpr int O_TAB = O_P + 2 * YS_B;
-  // gather tables, each face's list padded to whole 4-node groups
-  static constexpr int TAB_B = kMaxGather * 4 * FG;
+  // gather tables, each face's list padded to whole units
+  static constexpr int TAB_B = kMaxGather * FN * FG;
   static constexpr int SMEM = O_TAB + tc_r128(TAB_B);
   static_assert(SMEM <= 232448 - 1024, "shared memory per CTA (dynamic + static)");
   static_assert(T_ALO + KV <= TMEM_COLS, "TMEM columns");
@@ -268,18 +267,10 @@ __device__ __forceinline__ void tc_row_st(float* row, int i0, bool on, const flo
 // bounds a wait at about 2.1 s of wall time.  (A wall-clock check inside the
 // loop was tried: any extra state in these inlined loops slows the stage
 // kernel by 7 %.)
-#ifdef DGTD_TC_PHASE_TIMERS
-__device__ unsigned long long g_tc_polls[3];
-#endif
 __device__ __forceinline__ bool tc_wait1(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                          uint32_t limit = kTcWaitLimit) {
   for (uint32_t i = 0; i < limit; ++i) {
     if (tc::mbar_try_wait(bar, parity)) {
-#ifdef DGTD_TC_PHASE_TIMERS
-      const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-      if (l == 0 && (w == 0 || w == kTcVolWarp || w == kTcFluxWarp))
-        atomicAdd(&g_tc_polls[w == 0 ? 0 : w == kTcVolWarp ? 1 : 2], (unsigned long long)(i + 1));
-#endif
       return true;
     }
     if ((i & 255u) == 255u && *abort_flag) return false;
@@ -315,7 +306,7 @@ __global__ void __launch_bounds__(TcCfg<N>::THREADS, 1)
 rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   using C = TcCfg<N>;
   constexpr int NP = C::NP, NFP = C::NFP, E = C::E, M = C::M;
-  constexpr int KV = C::KV, NV = C::NV, KLF = C::KLF, NL = C::NL, FG = C::FG;
+  constexpr int KV = C::KV, NV = C::NV, KLF = C::KLF, NL = C::NL, FG = C::FG, FN = C::FN;
   extern __shared__ __align__(1024) unsigned char tsm[];
   __shared__ uint32_t s_tmem;
   __shared__ __align__(8) uint64_t bar_ld[3];   // state + records of a slot landed
@@ -330,8 +321,8 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   volatile int* const abort_flag = &s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool is_epi = warp < kTcEpiWarps;
-  const bool is_vol = !is_epi && warp < kTcFluxWarp;
+  const bool is_epi = warp < C::EPI_WARPS;
+  const bool is_vol = !is_epi && warp < C::FLUX_WARP;
   const bool is_flux = !is_epi && !is_vol && warp < C::CTL_WARP;
   const bool ctl0 = warp == C::CTL_WARP && lane == 0;
   const bool copy0 = warp == C::COPY_WARP && lane == 0;
@@ -354,9 +345,9 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&bar_p[i], 1);
       tc::mbar_init(&bar_mma[i], 1);
-      tc::mbar_init(&bar_epi[i], kTcEpiWarps);
+      tc::mbar_init(&bar_epi[i], C::EPI_WARPS);
     }
-    tc::mbar_init(&bar_avol, kTcVolWarps);
+    tc::mbar_init(&bar_avol, C::VOL_WARPS);
     tc::mbar_init(&bar_alift[0], C::WARPS_H);
     tc::mbar_init(&bar_alift[1], C::WARPS_H);
     tc::mbar_init(&bar_l0done, 1);
@@ -378,9 +369,9 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       reinterpret_cast<uint4*>(alh)[i] = make_uint4(0, 0, 0, 0);
       reinterpret_cast<uint4*>(all)[i] = make_uint4(0, 0, 0, 0);
     }
-    for (int i = tid; i < T.n_gather * 4 * FG; i += C::THREADS) {
-      const int m = tc_face_node<N>(i % (4 * FG));
-      sG[i] = m < NFP ? T.gtab[(i / (4 * FG)) * NFP + m] : (uint8_t)0;
+    for (int i = tid; i < T.n_gather * FN * FG; i += C::THREADS) {
+      const int m = tc_face_node(N, i % (FN * FG));
+      sG[i] = m < NFP ? T.gtab[(i / (FN * FG)) * NFP + m] : (uint8_t)0;
     }
   }
   tc::fence_proxy_async_smem();
@@ -396,7 +387,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
                            : 0;
 
 #ifdef DGTD_TC_PHASE_TIMERS
-  const bool timer_thread = lane == 0 && (warp == 0 || warp == kTcVolWarp || warp == kTcFluxWarp || warp >= C::CTL_WARP);
+  const bool timer_thread = lane == 0 && (warp == 0 || warp == C::VOL_WARP || warp == C::FLUX_WARP || warp >= C::CTL_WARP);
   unsigned long long clk_acc[kTcMarks] = {0};
   long long clk_last = clock64();
 #endif
@@ -485,22 +476,23 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
     // ================= flux warps: numerical fluxes -> LIFT operand
     // This thread's flux unit: node group mg (tc_face_node) of face f of element
     // le.  One unit per thread and tile: what belongs to the face (normal,
-    // scale, neighbour, face code) is read once for four nodes, and the four
-    // nodes of a row are one 16-byte vector of the LIFT operand.  The lanes of a
-    // face are neighbours, so a load of an out-of-tile trace touches few cache
-    // lines (neighbouring elements in neighbouring lanes: 28.1 against 21.3 ms
-    // for five 48^3 order-4 steps).
-    const int hh = (warp - kTcFluxWarp) / C::WARPS_H;  // half of the LIFT operand
-    const int uh = tid - (kTcFluxWarp + hh * C::WARPS_H) * 32;
+    // scale, neighbour, face code) is read once for FN nodes, and the nodes of a
+    // row are one vector of the LIFT operand.  The lanes of a face are
+    // neighbours, so a load of an out-of-tile trace touches few cache lines
+    // (neighbouring elements in neighbouring lanes: 28.1 against 21.3 ms for
+    // five 48^3 order-4 steps).
+    const int hh = (warp - C::FLUX_WARP) / C::WARPS_H;  // half of the LIFT operand
+    const int uh = tid - (C::FLUX_WARP + hh * C::WARPS_H) * 32;
     const bool has_unit = uh < C::UNITS_H;
     const int mg = uh % FG, le = (uh / FG) % E, f = (2 * hh + uh / (FG * E)) & 3;
-    int own[4];  // offsets of the nodes' states in the tile (component 0)
+    int own[FN];  // offsets of the nodes' states in the tile (component 0)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int m = tc_face_node<N>(4 * mg + i);
+    for (int i = 0; i < FN; ++i) {
+      const int m = tc_face_node(N, FN * mg + i);
       own[i] = le * 6 * NP + (has_unit && m < NFP ? (int)T.fnodes[f * NFP + m] : 0);
     }
-    const uint32_t a_off = (uint32_t)((f * (KLF / 4) + mg) * C::AL_CH + (le / C::EQ) * C::QR * 16);
+    const uint32_t a_off = (uint32_t)((f * (KLF / 4) + FN * mg / 4) * C::AL_CH + (FN * mg % 4) * 4 +
+                                      (le / C::EQ) * C::QR * 16);
     int ys = 0;
     uint32_t ld_par = 0u;  // bit s: parity of the next wait on bar_ld[s]
     for (int64_t it = 0; it < n_my; ++it) {
@@ -512,9 +504,9 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       DGTD_TC_MARK(8);
       // The neighbour's traces at the unit's nodes, as pairs of nodes: from the
       // tile in shared memory when the neighbour is in it, else from L2.
-      float tr[4][6];
+      float tr[FN][6];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < FN; ++i)
 #pragma unroll
         for (int c = 0; c < 6; ++c) tr[i][c] = 0.f;
       bool port = false;
@@ -523,28 +515,30 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
         const uint32_t code = reinterpret_cast<const uint16_t*>(Me + 41)[f];
         const int kind = (int)(code >> 8) & 3;
         if (kind == kInterior) {
-          const uint32_t g4 = reinterpret_cast<const uint32_t*>(sG)[(code & 0xff) * FG + mg];
+          int gn[FN];  // the neighbour's nodes
+          if constexpr (FN == 4) {
+            const uint32_t g = reinterpret_cast<const uint32_t*>(sG)[(code & 0xff) * FG + mg];
+#pragma unroll
+            for (int i = 0; i < FN; ++i) gn[i] = (g >> (8 * i)) & 0xff;
+          } else {
+            const uint32_t g = reinterpret_cast<const uint16_t*>(sG)[(code & 0xff) * FG + mg];
+            gn[0] = g & 0xff;
+            gn[1] = g >> 8;
+          }
           const int nbr = __float_as_int(Me[37 + f]);
           const int lo = nbr - (int)e0;  // element ids fit in int
-          const int g0 = g4 & 0xff, g1 = (g4 >> 8) & 0xff, g2 = (g4 >> 16) & 0xff, g3 = g4 >> 24;
           if ((uint32_t)lo < (uint32_t)E) {
             const float* Z = sY + lo * 6 * NP;
 #pragma unroll
-            for (int c = 0; c < 6; ++c) {
-              tr[0][c] = Z[g0 + c * NP];
-              tr[1][c] = Z[g1 + c * NP];
-              tr[2][c] = Z[g2 + c * NP];
-              tr[3][c] = Z[g3 + c * NP];
-            }
+            for (int c = 0; c < 6; ++c)
+#pragma unroll
+              for (int i = 0; i < FN; ++i) tr[i][c] = Z[gn[i] + c * NP];
           } else {
             const float* Z = P.y_in + (int64_t)nbr * (6 * NP);
 #pragma unroll
-            for (int c = 0; c < 6; ++c) {
-              tr[0][c] = __ldg(Z + g0 + c * NP);
-              tr[1][c] = __ldg(Z + g1 + c * NP);
-              tr[2][c] = __ldg(Z + g2 + c * NP);
-              tr[3][c] = __ldg(Z + g3 + c * NP);
-            }
+            for (int c = 0; c < 6; ++c)
+#pragma unroll
+              for (int i = 0; i < FN; ++i) tr[i][c] = __ldg(Z + gn[i] + c * NP);
           }
         } else if (kind == kPec) {
           // PEC ghost: [E] = 2 E_tan, [H] = 2 H_n (rhs.rs:1387-1402).  Both
@@ -553,10 +547,8 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
 #pragma unroll
           for (int c = 0; c < 6; ++c) {
             const float sg = c < 3 ? -1.f : 1.f;
-            tr[0][c] = sg * sY[own[0] + c * NP];
-            tr[1][c] = sg * sY[own[1] + c * NP];
-            tr[2][c] = sg * sY[own[2] + c * NP];
-            tr[3][c] = sg * sY[own[3] + c * NP];
+#pragma unroll
+            for (int i = 0; i < FN; ++i) tr[i][c] = sg * sY[own[i] + c * NP];
           }
         } else {
           port = true;  // characteristic boundary against a zero incident field (rhs.rs:1380-1386)
@@ -587,7 +579,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
         const uint64_t ax = tc::dup2(a * nx), ay = tc::dup2(a * ny), az = tc::dup2(a * nz);
         const uint64_t ca = tc::dup2(-coef * a);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < FN / 2; ++i) {
           const float* Y0 = sY + own[2 * i];
           const float* Y1 = sY + own[2 * i + 1];
           const uint64_t ex = tc::sub2(tc::pack2(tr[2 * i][0], tr[2 * i + 1][0]), tc::pack2(Y0[0 * NP], Y1[0 * NP]));
@@ -612,16 +604,21 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
           const uint32_t off = a_off + (uint32_t)(((C::EQ * c + le) & (C::QR - 1)) * 16);
-          float h[4], l[4];
+          float h[FN], l[FN];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
+          for (int i = 0; i < FN; ++i) {
             // the operand's padding columns stay zero whatever the fields hold
-            if (tc_face_node<N>(4 * (FG - 1) + i) >= NFP && tc_face_node<N>(4 * mg + i) >= NFP) tr[i][c] = 0.f;
+            if (tc_face_node(N, FN * (FG - 1) + i) >= NFP && tc_face_node(N, FN * mg + i) >= NFP) tr[i][c] = 0.f;
             h[i] = tc::tf32_round(tr[i][c]);
             l[i] = tr[i][c] - h[i];
           }
-          *reinterpret_cast<float4*>(alh + off) = make_float4(h[0], h[1], h[2], h[3]);
-          *reinterpret_cast<float4*>(all + off) = make_float4(l[0], l[1], l[2], l[3]);
+          if constexpr (FN == 4) {
+            *reinterpret_cast<float4*>(alh + off) = make_float4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<float4*>(all + off) = make_float4(l[0], l[1], l[2], l[3]);
+          } else {
+            *reinterpret_cast<float2*>(alh + off) = make_float2(h[0], h[1]);
+            *reinterpret_cast<float2*>(all + off) = make_float2(l[0], l[1]);
+          }
         }
       }
       tc::fence_proxy_async_smem();
@@ -693,7 +690,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
       constexpr int kUnits = C::LANE_SETS ? C::EPAIRS : C::ECH;
 #pragma unroll
       for (int cc = 0; cc < kIters; ++cc) {
-        const int ch = eg + kTcEpiGroups * cc;
+        const int ch = eg + C::EPI_GROUPS * cc;
         if (ch < kUnits) {
           const int c0 = C::LANE_SETS ? ch * 8 : ch * 4;  // first column of the access
           const int i0 = c0 + (hb >> 2);                  // this thread's first node
