@@ -4,11 +4,11 @@
 //
 // One persistent CTA per SM walks tiles of E elements.  The MMA M dimension is
 // the rows (element, component), split into four lane quarters of QR = M/4
-// rows; quarter q holds elements EQ q .. EQ q + EQ - 1, component c of the
-// tile's element e in row QR q + (EQ c + e) mod QR, so the six components of an
-// element sit in one warp's TMEM lanes and the curl can be combined with warp
-// shuffles, and eight neighbouring elements' rows of one component differ
-// mod 8 (conflict-free 16-byte stores of the LIFT operand).
+// rows; quarter q holds elements EQ q .. EQ q + EQ - 1, component by component
+// (tc_row_in_quarter), so the six components of an element sit in one warp's TMEM
+// lanes and the curl can be combined with warp shuffles, and neighbouring
+// elements' rows of one component differ mod 8 (16-byte stores of the LIFT
+// operand without replays).
 //   orders 1-4: M = 128, EQ = 5 (E = 20; rows 30, 31 of a quarter are padding),
 //               two TMEM accumulator sets side by side in the columns;
 //   order 5:    M = 64, EQ = 2 (E = 8; rows 12..15 of a quarter are padding).
@@ -41,18 +41,19 @@
 // The LIFT operand is formed and multiplied in two halves (faces 0-1, 2-3) by
 // separate warps, each half released by its own MMA completion.
 //
-// What bounds it: the flux warps' chain of one tile (trace loads, fluxes, operand
-// stores) and the epilogue's are both nearly as long as the tile period, with
-// the load/store pipe 60 % busy; HBM and the tensor pipe are not.  One thread per
-// (element, face, four nodes) with 16-byte operand stores, the loads of a face
-// in neighbouring lanes, packed f32x2 arithmetic, a copy lane that refills a
-// slot as soon as it is read and volume warps of their own took five order-4
-// steps of the 48^3 box from 21.7 to 18.1 ms, twenty order-3 steps of the graded
-// 24^3 box from 10.6 to 8.1 ms, ten order-5 steps of 14,586 elements from 2.86
-// to 2.15 ms (one node per thread, 4-byte stores, the flux warps also writing
-// the volume operand, copies issued between the MMAs).  Loading a tile's
-// out-of-tile traces while the previous tile's fluxes are formed measured
-// slower (8, 6 and 4 % more).
+// What bounds it: at order 4 the flux warps' chain of one tile (trace loads,
+// fluxes, operand stores), nearly as long as the tile period, with the
+// load/store pipe about 70 % busy; at order 3 that pipe, 86 % busy before the row
+// order below, a third of it replays of the face-node reads.  HBM and the tensor
+// pipe (18 to 24 %) are not.  One thread per (element, face, node group) with
+// vector operand stores, the loads of a face in neighbouring lanes, packed f32x2
+// arithmetic, a copy lane that refills a slot as soon as it is read and volume
+// warps of their own took five order-4 steps of the 48^3 box from 21.7 to 18.1
+// ms, twenty order-3 steps of the graded 24^3 box from 10.6 to 8.1 ms, ten
+// order-5 steps of 14,586 elements from 2.86 to 2.15 ms (one node per thread,
+// 4-byte stores, the flux warps also writing the volume operand, copies issued
+// between the MMAs).  Loading a tile's out-of-tile traces while the previous
+// tile's fluxes are formed measured slower (8, 6 and 4 % more).
 // All hand-offs are mbarriers; every wait is bounded and an expired wait stops
 // the CTA cleanly with an error flag.  The element count is padded on the
 // device to a multiple of E with inert records (PEC faces, zero metric), so
@@ -162,6 +163,7 @@ struct TcCfg {
   static constexpr int FLUX_WARP = VOL_WARP + VOL_WARPS;
   static constexpr int CTL_WARP = FLUX_WARP + 2 * WARPS_H, COPY_WARP = CTL_WARP + 1;
   static constexpr int THREADS = (COPY_WARP + 1) * 32;
+  static constexpr bool SLOT4 = N == 3;                                        // see tc_row_in_quarter
   static constexpr bool VEC = NP % 4 == 0;                                     // state rows are whole 16-byte vectors
   static constexpr int KS_H = KL / 16;                                         // LIFT k-steps per half
   static constexpr int VCH = KV / 8;                                           // volume-operand column chunks
@@ -220,17 +222,37 @@ __device__ __forceinline__ uint32_t tc_set_off(int s) {
   return C::LANE_SETS ? ((uint32_t)(16 * s) << 16) : (uint32_t)(s * C::ACC);
 }
 
-// MMA row of (element le, component c) of a tile.
+// MMA row of (element le, component c) of a tile: slot EQ c + el of the element's
+// lane quarter, rotated by EQ times the quarter.  At order 3 the slots are 4 c + el
+// of the quarter's first four elements, then 24 + c of its fifth, rotated by 4 in
+// the odd quarters: the state rows (5 c + 30 el 16-byte units) of eight neighbouring
+// lanes then fall into eight bank groups, which the 16-byte accesses of the
+// epilogue and the volume warps need, and the operand stores lose nothing (82,944
+// elements: 70.7 -> 68.4 us per stage).  Padding the elements apart in shared
+// memory instead, at the price of one bulk copy per element, measured 99 us.
 template <class C>
-__device__ __forceinline__ int tc_row(int le, int c) {
-  return (le / C::EQ) * C::QR + ((C::EQ * c + le) & (C::QR - 1));
+__device__ __forceinline__ int tc_rot(int q) {
+  return C::SLOT4 ? 4 * (q & 1) : C::EQ * q;
+}
+template <class C>
+__device__ __forceinline__ int tc_row_in_quarter(int le, int c) {
+  const int q = le / C::EQ, el = le - q * C::EQ;
+  const int slot = !C::SLOT4 ? C::EQ * c + el : el < 4 ? 4 * c + el : 24 + c;
+  return (slot + tc_rot<C>(q)) & (C::QR - 1);
 }
 
-// The (element in quarter, component) of a row r of quarter q: EQ c + el, or a
-// value >= RL for a padding row.
+// The slot of row r of quarter q (>= RL: a padding row), and what it holds.
 template <class C>
 __device__ __forceinline__ int tc_row_slot(int q, int r) {
-  return (r - C::EQ * q) & (C::QR - 1);
+  return (r - tc_rot<C>(q)) & (C::QR - 1);
+}
+template <class C>
+__device__ __forceinline__ int tc_slot_el(int s) {
+  return !C::SLOT4 ? s % C::EQ : s < 24 ? s & 3 : 4;
+}
+template <class C>
+__device__ __forceinline__ int tc_slot_comp(int s) {
+  return !C::SLOT4 ? s / C::EQ : s < 24 ? s >> 2 : s - 24;
 }
 
 // Nodes i0 .. i0 + 3 of a state row in shared or global memory (one 16-byte access where
@@ -238,7 +260,8 @@ __device__ __forceinline__ int tc_row_slot(int q, int r) {
 template <class C>
 __device__ __forceinline__ void tc_row_ld(const float* row, int i0, bool on, float (&v)[4]) {
   if constexpr (C::VEC) {
-    const float4 t = *reinterpret_cast<const float4*>(row + i0);  // a padding lane reads its clamped row
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (on) t = *reinterpret_cast<const float4*>(row + i0);
     v[0] = t.x;
     v[1] = t.y;
     v[2] = t.z;
@@ -399,7 +422,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
     // lane & 15 of the set's lane half, the thread half choosing the columns
     const int v_slot = tc_row_slot<C>(q4, lane & (C::QR - 1));
     const bool lane_real = v_slot < C::RL;
-    const int v_src = lane_real ? ((q4 * C::EQ + v_slot % C::EQ) * 6 + v_slot / C::EQ) * NP : 0;
+    const int v_src = lane_real ? ((q4 * C::EQ + tc_slot_el<C>(v_slot)) * 6 + tc_slot_comp<C>(v_slot)) * NP : 0;
     const uint32_t v_taddr = tmem + ((uint32_t)(q4 * 32) << 16);
     int ys = 0;
     uint32_t ld_par = 0u;  // bit s: parity of the next wait on bar_ld[s]
@@ -603,7 +626,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
         // 2^-22-class terms in the sum of many products.
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-          const uint32_t off = a_off + (uint32_t)(((C::EQ * c + le) & (C::QR - 1)) * 16);
+          const uint32_t off = a_off + (uint32_t)(tc_row_in_quarter<C>(le, c) * 16);
           float h[FN], l[FN];
 #pragma unroll
           for (int i = 0; i < FN; ++i) {
@@ -635,11 +658,11 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
     const int hb = C::LANE_SETS ? (lane & 16) : 0;
     const int e_slot = tc_row_slot<C>(q4, lane & (C::QR - 1));
     const bool lane_real = e_slot < C::RL;
-    const int e_el = lane_real ? e_slot % C::EQ : C::EQ - 1, e_c = lane_real ? e_slot / C::EQ : 5;
+    const int e_el = lane_real ? tc_slot_el<C>(e_slot) : C::EQ - 1, e_c = lane_real ? tc_slot_comp<C>(e_slot) : 5;
     const int e_le = q4 * C::EQ + e_el;
     const int e_fld = e_c / 3, e_t = e_c % 3;
-    const int e_srcA = hb + ((C::EQ * (3 * (1 - e_fld) + (e_t + 2) % 3) + e_le) & (C::QR - 1));
-    const int e_srcB = hb + ((C::EQ * (3 * (1 - e_fld) + (e_t + 1) % 3) + e_le) & (C::QR - 1));
+    const int e_srcA = hb + tc_row_in_quarter<C>(e_le, 3 * (1 - e_fld) + (e_t + 2) % 3);
+    const int e_srcB = hb + tc_row_in_quarter<C>(e_le, 3 * (1 - e_fld) + (e_t + 1) % 3);
     const float e_sign = e_fld == 0 ? 1.f : -1.f;
     const int e_cA = (e_t + 2) % 3, e_cB = (e_t + 1) % 3;
     const int e_row_off = (e_le * 6 + e_c) * NP;
