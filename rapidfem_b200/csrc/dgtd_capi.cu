@@ -349,9 +349,14 @@ int to_aos(dgtd_op* op, const TI* soa, TO* aos) {
 // ---- RHS kernel dispatch
 template <int N, int MODE, int TD>
 int launch_rhs_n(dgtd_op* op, const RhsParams& P) {
-  using C = Fp32Cfg<N, float, TD>;
+  using C = CcCfg<N, float, TD>;
   static int blocks_per_sm[8] = {0};
-  auto kern = rhs_fp32_kernel<N, MODE, TD>;
+  const auto kern = [] {
+    if constexpr (N == 4)
+      return rhs_fp32_pair_kernel<N, MODE, TD>;
+    else
+      return rhs_fp32_kernel<N, MODE, TD>;
+  }();
   int& bps = blocks_per_sm[op->ctx->device & 7];
   if (bps == 0) {
     CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
@@ -369,9 +374,14 @@ int launch_rhs_n(dgtd_op* op, const RhsParams& P) {
 
 template <int N, int MODE>
 int launch_rhs64_n(dgtd_op* op, const RhsParamsT<double>& P) {
-  using C = Fp32Cfg<N, double>;
+  using C = CcCfg<N, double>;
   static int blocks_per_sm[8] = {0};
-  auto kern = rhs_fp64_kernel<N, MODE>;
+  const auto kern = [] {
+    if constexpr (N == 4)
+      return rhs_fp64_pair_kernel<N, MODE>;
+    else
+      return rhs_fp64_kernel<N, MODE>;
+  }();
   int& bps = blocks_per_sm[op->ctx->device & 7];
   if (bps == 0) {
     CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));

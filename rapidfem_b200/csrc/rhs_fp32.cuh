@@ -18,8 +18,10 @@
 // D and LIFT live in shared memory for the whole kernel.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "dgtd_common.cuh"
+#include "tc_util.cuh"
 
 namespace dgtd {
 
@@ -351,6 +353,348 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
   // Several of these CTAs share an SM: a next launch let in earlier is placed
   // wherever there is room, unevenly (the f64 kernel: 13 % slower).
   pdl_launch();
+}
+
+// The numerical flux (rhs.rs:1370-1441) at the face nodes of a tile's `ne` elements
+// from e0 on, by all threads: states sY and fluxes sF with element strides YS, FS.
+// (As in rhs_cc_body, which keeps its own copy: called from there it cost order 5
+// 18 %.)
+template <int N, int YS, int FS, class R>
+__device__ __forceinline__ void rhs_cc_flux(const RhsParamsT<R>& P, int64_t e0, int ne, const R* sY, const R* sM,
+                                            const uint8_t* sFn, const uint8_t* sG, R* sF) {
+  constexpr int NP = np_of(N), NFP = nfp_of(N), NF = 4 * NFP;
+  for (int q = threadIdx.x; q < ne * NF; q += blockDim.x) {
+    const int le = q / NF;
+    const int s = q - le * NF;
+    const int f = s / NFP;
+    const int m = s - f * NFP;
+    const R* M = sM + le * kMetaWords;
+    const R nx = M[9 + 3 * f], ny = M[10 + 3 * f], nz = M[11 + 3 * f];
+    const R coef = R(0.5) * M[21 + f];
+    const int nbr = rec_int(M[37 + f]);
+    const uint32_t codes = rec_uint(M[41 + (f >> 1)]);
+    const uint32_t code = (f & 1) ? (codes >> 16) : (codes & 0xffffu);
+    const int kind = (code >> 8) & 3;
+    const int vi = sFn[f * NFP + m];
+    const R* Y = sY + le * YS;
+    const R ex = Y[0 * NP + vi], ey = Y[1 * NP + vi], ez = Y[2 * NP + vi];
+    const R hx = Y[3 * NP + vi], hy = Y[4 * NP + vi], hz = Y[5 * NP + vi];
+    R jex, jey, jez, jhx, jhy, jhz;
+    R a = P.alpha;
+    if (kind == kPort) {
+      // characteristic boundary against a zero incident field (rhs.rs:1380-1386)
+      jex = ex; jey = ey; jez = ez; jhx = hx; jhy = hy; jhz = hz;
+      a = R(1);
+    } else if (kind == kPec) {
+      // PEC ghost: [E] = 2 E_tan, [H] = 2 H_n (rhs.rs:1387-1402)
+      const R edn = nx * ex + ny * ey + nz * ez;
+      const R hdn = nx * hx + ny * hy + nz * hz;
+      jex = R(2) * (ex - edn * nx); jey = R(2) * (ey - edn * ny); jez = R(2) * (ez - edn * nz);
+      jhx = R(2) * (hdn * nx); jhy = R(2) * (hdn * ny); jhz = R(2) * (hdn * nz);
+    } else {
+      const int vj = sG[(code & 0xff) * NFP + m];
+      const int64_t lo = (int64_t)nbr - e0;
+      R px, py, pz, qx, qy, qz;
+      if (lo >= 0 && lo < ne) {
+        const R* Z = sY + lo * YS;
+        px = Z[0 * NP + vj]; py = Z[1 * NP + vj]; pz = Z[2 * NP + vj];
+        qx = Z[3 * NP + vj]; qy = Z[4 * NP + vj]; qz = Z[5 * NP + vj];
+      } else {
+        const R* Z = P.y_in + (int64_t)nbr * 6 * NP;
+        px = __ldg(Z + 0 * NP + vj); py = __ldg(Z + 1 * NP + vj); pz = __ldg(Z + 2 * NP + vj);
+        qx = __ldg(Z + 3 * NP + vj); qy = __ldg(Z + 4 * NP + vj); qz = __ldg(Z + 5 * NP + vj);
+      }
+      jex = ex - px; jey = ey - py; jez = ez - pz;
+      jhx = hx - qx; jhy = hy - qy; jhz = hz - qz;
+    }
+    // n x [H], n x [E], n x (n x [E]), n x (n x [H])   (rhs.rs:1420-1432)
+    R nhx, nhy, nhz, nex, ney, nez, pex, pey, pez, phx, phy, phz;
+    cross3f(nx, ny, nz, jhx, jhy, jhz, nhx, nhy, nhz);
+    cross3f(nx, ny, nz, jex, jey, jez, nex, ney, nez);
+    cross3f(nx, ny, nz, nex, ney, nez, pex, pey, pez);
+    cross3f(nx, ny, nz, nhx, nhy, nhz, phx, phy, phz);
+    R* F = sF + le * FS;
+    F[0 * NF + s] = coef * (-nhx + a * pex);
+    F[1 * NF + s] = coef * (-nhy + a * pey);
+    F[2 * NF + s] = coef * (-nhz + a * pez);
+    F[3 * NF + s] = coef * (nex + a * phx);
+    F[4 * NF + s] = coef * (ney + a * phy);
+    F[5 * NF + s] = coef * (nez + a * phz);
+  }
+}
+
+template <class R> struct Vec2;
+template <> struct Vec2<float> { using T = float2; };
+template <> struct Vec2<double> { using T = double2; };
+
+// The two nodes of a thread (an f32 pair or two f64): x += a * v for a row of
+// operator entries a (one vector load) and one value v.
+template <class R> struct Acc;
+template <> struct Acc<float> {
+  uint64_t p;
+  using Row = uint64_t;
+  using Val = uint64_t;
+  __device__ __forceinline__ void zero() { p = 0ull; }
+  __device__ __forceinline__ static Row row(const float* s) { return *reinterpret_cast<const uint64_t*>(s); }
+  __device__ __forceinline__ static Val val(float v) { return tc::dup2(v); }
+  __device__ __forceinline__ void fma(Row a, Val v) { p = tc::fma2(a, v, p); }
+  __device__ __forceinline__ void get(float (&o)[2]) const { tc::unpack2(p, o[0], o[1]); }
+  __device__ __forceinline__ void set(const float (&o)[2]) { p = tc::pack2(o[0], o[1]); }
+};
+template <> struct Acc<double> {
+  double p[2];
+  using Row = double2;
+  using Val = double;
+  __device__ __forceinline__ void zero() { p[0] = p[1] = 0.0; }
+  __device__ __forceinline__ static Row row(const double* s) { return *reinterpret_cast<const double2*>(s); }
+  __device__ __forceinline__ static Val val(double v) { return v; }
+  __device__ __forceinline__ void fma(const Row& a, Val v) {
+    p[0] = ::fma(a.x, v, p[0]);
+    p[1] = ::fma(a.y, v, p[1]);
+  }
+  __device__ __forceinline__ void get(double (&o)[2]) const { o[0] = p[0]; o[1] = p[1]; }
+  __device__ __forceinline__ void set(const double (&o)[2]) { p[0] = o[0]; p[1] = o[1]; }
+};
+
+// Order 4: two nodes per thread.  The other orders' bodies own one node per thread;
+// their contractions wait for shared memory (9 loads per 18 multiply-adds).  Here
+// a thread's nodes are NG apart, so neighbouring threads hold neighbouring nodes
+// (coalesced global accesses), and next to each other in the shared D and LIFT
+// rows: one vector load brings a row entry for both, a state or flux value is
+// read once for both, and f32 arithmetic is packed (f32x2).  48,000 elements:
+// 219 -> 173 us per f32 stage (TD = 2: 230 -> 180); f64, 10,368 elements: 1.26
+// times faster.  Not at the other orders, where the fluxes are the larger part and
+// half the threads form them: order 3 76 -> 75 us (1,296 elements: 9.2 -> 13.0),
+// order 2 59 -> 66, order 1 32 -> 43, order 5 193 -> 193 (f64: order 3 18.7 ->
+// 21.4 ms, order 5 23.7 -> 23.4, orders 1 and 2 the same).
+template <int N, class R, int TD>
+struct PairCfg {
+  static constexpr bool F32 = sizeof(R) == 4;
+  static constexpr int NP = np_of(N), NFP = nfp_of(N), NF = 4 * NFP;
+  static constexpr int NPT = 2, NG = (NP + 1) / 2, NPAD = NPT * NG;
+  // Elements per tile (TD = 2: half as many); all threads form fluxes, the
+  // first E * NG own nodes.
+  static constexpr int E = F32 ? 14 / TD : 12;
+  static constexpr int OWNERS = E * NG;
+  static constexpr int THREADS = OWNERS < 256 / TD ? 256 / TD : (OWNERS + 31) / 32 * 32;
+  // element strides (in R) of the state and flux tiles: the elements of a warp in
+  // different banks, flux rows whole 16-byte vectors
+  static constexpr int YS = 6 * NP + (F32 ? 0 : 2), FS = 6 * NF + 4;
+  static constexpr int PER16 = 16 / (int)sizeof(R);
+  static constexpr int al4(int x) { return (x + PER16 - 1) / PER16 * PER16; }
+  static constexpr int OFF_D = 0;
+  static constexpr int OFF_L = al4(OFF_D + 3 * NP * NPAD);
+  static constexpr int OFF_Y = al4(OFF_L + NF * NPAD);
+  static constexpr int OFF_F = al4(OFF_Y + E * YS);
+  static constexpr int OFF_M = al4(OFF_F + E * FS);
+  static constexpr int OFF_B = al4(OFF_M + E * kMetaWords);
+  static constexpr int BYTES_TAB = 4 * NFP + kMaxGather * NFP;
+  static constexpr int SMEM = OFF_B * (int)sizeof(R) + ((BYTES_TAB + 15) / 16) * 16;
+  static_assert(FS % PER16 == 0 && NF % PER16 == 0, "flux rows are whole vectors");
+  static_assert(YS % 2 == 0 && (6 * NP) % 2 == 0, "the state is copied in pairs");
+  static_assert((kMetaWords % PER16) == 0, "element records are whole 16-byte vectors");
+};
+
+template <int N, int MODE, class R, int TD = 1>
+__device__ __forceinline__ void rhs_cc_pair_body(const RhsParamsT<R>& P, const OpTablesT<R>& T) {
+  using C = PairCfg<N, R, TD>;
+  using V = typename Vec16<R>::T;
+  using A = Acc<R>;
+  constexpr int NP = C::NP, NFP = C::NFP, NF = C::NF, E = C::E, NPT = C::NPT, NG = C::NG, NPAD = C::NPAD;
+  constexpr int YS = C::YS, FS = C::FS;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  R* smem = reinterpret_cast<R*>(smem_raw);
+  R* sD = smem + C::OFF_D;
+  R* sL = smem + C::OFF_L;
+  R* sY = smem + C::OFF_Y;
+  R* sF = smem + C::OFF_F;
+  R* sM = smem + C::OFF_M;
+  uint8_t* sFn = reinterpret_cast<uint8_t*>(smem + C::OFF_B);
+  uint8_t* sG = sFn + 4 * NFP;
+  const int tid = threadIdx.x;
+
+  // rows of NPAD: entry NPT g + q is node g + NG q (zero past the last node)
+  for (int i = tid; i < (3 * NP + NF) * NPAD; i += blockDim.x) {
+    const int row = i / NPAD, x = i - row * NPAD, node = x / NPT + NG * (x % NPT);
+    const R* src = row < 3 * NP ? T.dT + row * NP : T.liftT + (row - 3 * NP) * NP;
+    (row < 3 * NP ? sD + i : sL + i - 3 * NP * NPAD)[0] = node < NP ? src[node] : R(0);
+  }
+  for (int i = tid; i < 4 * NFP; i += blockDim.x) sFn[i] = T.fnodes[i];
+  for (int i = tid; i < T.n_gather * NFP; i += blockDim.x) sG[i] = T.gtab[i];
+
+  pdl_wait();
+  if (P.skip != nullptr && *P.skip) return;  // uniform: nothing to do for this launch
+  R kry_sig = 1, kry_g = 0;
+  if (MODE == kModeKrylov) {
+    kry_sig = (R)P.kry[0];
+    kry_g = (R)P.kry[1];
+  }
+
+  const int64_t n_tiles = (P.n_elem - P.e_begin + E - 1) / E;
+  const int le_me = tid / NG;
+  const int g_me = tid - le_me * NG;  // nodes g_me + NG q, q < NPT
+  const bool owns = tid < C::OWNERS;
+
+  for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const int64_t e0 = P.e_begin + tile * E;
+    const int ne = (int)((P.n_elem - e0) < E ? (P.n_elem - e0) : E);
+    __syncthreads();  // previous tile fully consumed (and tables loaded on the first pass)
+    // ---- 1. state tile and element records -> shared memory
+    {
+      using V2 = typename Vec2<R>::T;
+      const V2* src = reinterpret_cast<const V2*>(P.y_in + e0 * 6 * NP);
+      for (int i = tid; i < ne * (3 * NP); i += blockDim.x) {
+        const int el = i / (3 * NP);
+        *reinterpret_cast<V2*>(sY + el * YS + 2 * (i - el * (3 * NP))) = __ldg(src + i);
+      }
+    }
+    {
+      const V* m4 = reinterpret_cast<const V*>(P.meta + e0 * kMetaWords);
+      V* d4 = reinterpret_cast<V*>(sM);
+      for (int i = tid; i < ne * kMetaWords / C::PER16; i += blockDim.x) d4[i] = __ldg(m4 + i);
+    }
+    __syncthreads();
+
+    // ---- 2. numerical flux at the 4*Nfp face nodes of each element
+    rhs_cc_flux<N, YS, FS>(P, e0, ne, sY, sM, sFn, sG, sF);
+
+    // ---- 3. volume term: reference derivatives of E and H at my nodes
+    const bool active = owns && le_me < ne;
+    A dd[6];  // dE = curl H, dH = -curl E at the thread's nodes
+    if (active) {
+      const R* Y = sY + le_me * YS;
+      A r[3][6];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) r[k][c].zero();
+#pragma unroll 2
+      for (int j = 0; j < NP; ++j) {
+        typename A::Row d[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) d[k] = A::row(sD + (k * NP + j) * NPAD + NPT * g_me);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          const auto v = A::val(Y[c * NP + j]);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) r[k][c].fma(d[k], v);
+        }
+      }
+      // physical derivatives pd[p][c] = sum_k Jinv[k][p] r[k][c] (rhs.rs:62-75),
+      // dE = curl H, dH = -curl E (rhs.rs:78-84, :1365-1368)
+      const R* M = sM + le_me * kMetaWords;
+      R rv[3][6][NPT];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) r[k][c].get(rv[k][c]);
+      const auto pd = [&](int p, int c, int q) {
+        return M[0 * 3 + p] * rv[0][c][q] + M[1 * 3 + p] * rv[1][c][q] + M[2 * 3 + p] * rv[2][c][q];
+      };
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        const int a = (t + 1) % 3, b = (t + 2) % 3;
+        R de[NPT], dh[NPT];
+#pragma unroll
+        for (int q = 0; q < NPT; ++q) {
+          de[q] = pd(a, 3 + b, q) - pd(b, 3 + a, q);
+          dh[q] = -(pd(a, b, q) - pd(b, a, q));
+        }
+        dd[t].set(de);
+        dd[3 + t].set(dh);
+      }
+    }
+    __syncthreads();  // flux complete
+
+    // ---- 4. LIFT, materials, epilogue
+    if (active) {
+      const R* F = sF + le_me * FS;
+      constexpr int SV = C::PER16;  // face nodes per vector of a flux row
+#pragma unroll 1
+      for (int s0 = 0; s0 < NF; s0 += SV) {
+        typename A::Row w[SV];
+#pragma unroll
+        for (int ss = 0; ss < SV; ++ss) w[ss] = A::row(sL + (s0 + ss) * NPAD + NPT * g_me);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          const V fv = *reinterpret_cast<const V*>(F + c * NF + s0);
+          const R* f = reinterpret_cast<const R*>(&fv);
+#pragma unroll
+          for (int ss = 0; ss < SV; ++ss) dd[c].fma(w[ss], A::val(f[ss]));
+        }
+      }
+      const R* M = sM + le_me * kMetaWords;
+      const R* Y = sY + le_me * YS;
+      R kcl_h = 0, kcl_gs = 0;
+      if (MODE == kModeKcl) {
+        kcl_h = (R)*P.kcl_h;
+        kcl_gs = P.kcl_g != nullptr ? (R)P.kcl_g[*P.kcl_frame] : R(0);
+      }
+      const int64_t base = (e0 + le_me) * 6 * NP;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        R dv[NPT];
+        dd[c].get(dv);
+        const R mw = M[25 + c], ms = M[31 + c];
+#pragma unroll
+        for (int q = 0; q < NPT; ++q) {
+          const int i = g_me + NG * q;
+          if (i < NP) {
+            const int64_t g = base + c * NP + i;
+            const R yv = Y[c * NP + i];
+            const R dy = mw * dv[q] - ms * yv;
+            if (MODE == kModeApply) {
+              P.out[g] = dy;
+            } else if (MODE == kModeLserk) {
+              R k = dy;
+              if (P.src_vec != nullptr) k = fma(P.src_g, __ldg(P.src_vec + g), k);
+              if (g == P.src_idx) k += P.src_g;
+              R pv = (P.dt * M[43]) * k;
+              if (P.read_p) pv = fma(P.a, P.p[g], pv);
+              if (P.write_p) P.p[g] = pv;
+              P.out[g] = fma(P.b, pv, yv);
+            } else if (MODE == kModeKcl) {
+              // KCL stage (explicit_adaptive.rs:84-152), in the operation order of
+              // the separate stage kernel (kcl.cuh k_kcl_stage)
+              R kk = dy;
+              if (P.src_vec != nullptr) kk += P.src_vec[g] * kcl_gs;
+              if (g == P.src_idx) kk += kcl_gs;
+              const R f = kcl_h * kk;
+              const R yn = P.kcl_y[g] + P.kcl_b * f;
+              P.kcl_y[g] = yn;
+              P.kcl_e[g] = P.kcl_stage == 0 ? P.kcl_ew * f : P.kcl_e[g] + P.kcl_ew * f;
+              if (P.kcl_next != nullptr) P.kcl_next[g] = yn + P.kcl_amb * f;
+            } else {
+              // Krylov matvec of a stored basis vector: its scale and the source
+              // coefficient of the augmented system come from device memory
+              R w = kry_sig * dy;
+              if (P.src_vec != nullptr) w = fma(kry_g, __ldg(P.src_vec + g), w);
+              if (g == P.src_idx) w += kry_g;
+              P.out[g] = w;
+            }
+          }
+        }
+      }
+    }
+  }
+  // Several of these CTAs share an SM: a next launch let in earlier is placed
+  // wherever there is room, unevenly (the f64 kernel: 13 % slower).
+  pdl_launch();
+}
+
+template <int N, class R, int TD = 1>
+using CcCfg = std::conditional_t<N == 4, PairCfg<N, R, TD>, Fp32Cfg<N, R, TD>>;
+
+// Order 4 (three blocks per SM in f32, 80 registers).
+template <int N, int MODE, int TD = 1>
+__global__ void __launch_bounds__(PairCfg<N, float, TD>::THREADS, 3 * TD)
+rhs_fp32_pair_kernel(RhsParams P, OpTables T) {
+  rhs_cc_pair_body<N, MODE, float, TD>(P, T);
+}
+template <int N, int MODE>
+__global__ void __launch_bounds__(PairCfg<N, double, 1>::THREADS)
+rhs_fp64_pair_kernel(RhsParamsT<double> P, OpTablesT<double> T) {
+  rhs_cc_pair_body<N, MODE, double, 1>(P, T);
 }
 
 // FP32 engine (stage, RHS and the Krylov matvec of an f32 basis); TD = 2 is

@@ -122,3 +122,20 @@ def test_runs_on_two_streams(ctx):
     for _ in range(20):
         ops[0].run_lserk(1e-3, 5)
     assert np.array_equal(a, b) and np.array_equal(a, ops[0].download())
+
+
+@pytest.mark.parametrize("n_tets", [1, 6, 7, 8, 12, 13, 14, 15, 29, 360])
+def test_order_4_pairs_at_tile_edges(ctx, n_tets):
+    """The CUDA-core kernels of order 4 (two nodes per thread; tiles of 14, 7
+    and 12 elements) on rough fields; f64 to the rounding of the same sums."""
+    m, port, mat = _mixed_box(n_tets)
+    prod = O.MaxwellOperator(m, 4, 0.3, face_port=port, materials=mat)
+    orc = R.Operator(m.nodes, m.tets, 4, 0.3, face_port=port, materials=mat)
+    gop = G.GpuOperator(ctx, prod)
+    y = np.random.default_rng(4).standard_normal(gop.n_dof())
+    y32 = y.astype(np.float32)
+    want = orc.apply(y32.astype(np.float64))
+    for engine in (_native.ENGINE_FP32, _native.ENGINE_FP32_SMALL_TILES):
+        gop.set_engine(engine)
+        assert rel_l2(gop.apply(y32), want) < 5e-6
+    assert rel_l2(gop.apply_f64(y), orc.apply(y)) < 1e-11
