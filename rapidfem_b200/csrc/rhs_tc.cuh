@@ -361,7 +361,6 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
 
   // ---- set-up: TMEM, barriers, constant operands, tables (while the previous
   // launch still runs, on SMs that it leaves)
-  pdl_launch();
   if (warp == 0) tc::tmem_alloc(&s_tmem, C::TMEM_COLS);
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) tc::mbar_init(&bar_ld[i], 1);
@@ -402,6 +401,12 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = s_tmem;
+  // Only now, with this CTA's TMEM in hand: a CTA of the next launch that shared
+  // its SM could otherwise take the columns first and wait for this grid, which
+  // would wait for the columns, without a limit.  So a launch that waits for
+  // columns lets no other in, and one that lets others in has all its columns,
+  // whatever number of CTAs the compiler's register count lets an SM hold.
+  pdl_launch();
   pdl_wait();
   // a launch flagged off (adaptive stepping past its last attempt) has no tiles
   const bool off = P.skip != nullptr && *P.skip;
