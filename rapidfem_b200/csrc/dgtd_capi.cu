@@ -248,7 +248,7 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), unsigned grid, unsigned block, si
 // compile-time constant).
 constexpr int kRelayoutElems = 8;
 template <class TI, class TO, int NP, bool TO_SOA>
-__global__ void __launch_bounds__(256) k_relayout(const TI* __restrict__ src, TO* __restrict__ dst, int64_t n_elem) {
+__global__ void __launch_bounds__(256) k_relayout(const TI* src, TO* dst, int64_t n_elem) {
   constexpr int PER = 6 * NP, CH = kRelayoutElems * PER;
   __shared__ TI buf[CH];
   pdl_wait();
@@ -275,8 +275,7 @@ __global__ void __launch_bounds__(256) k_relayout(const TI* __restrict__ src, TO
   }
   pdl_launch();  // late: a stage kernel placed earlier takes a whole SM from the blocks still to come
 }
-__global__ void k_gather_f32(const float* __restrict__ src, const int64_t* __restrict__ idx,
-                             int64_t n, float* __restrict__ out) {
+__global__ void k_gather_f32(const float* src, const int64_t* __restrict__ idx, int64_t n, float* out) {
   pdl_launch();
   pdl_wait();
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
@@ -285,9 +284,9 @@ __global__ void k_gather_f32(const float* __restrict__ src, const int64_t* __res
 
 // One block per functional: sum_k w[k] * y[idx[k]] in f64 (fixed order per
 // thread and a fixed reduction tree, so the result is deterministic).
-__global__ void __launch_bounds__(256) k_functionals(const float* __restrict__ y, const int64_t* __restrict__ ptr,
+__global__ void __launch_bounds__(256) k_functionals(const float* y, const int64_t* __restrict__ ptr,
                                                      const int64_t* __restrict__ idx, const double* __restrict__ w,
-                                                     double* __restrict__ out) {
+                                                     double* out) {
   pdl_launch();
   pdl_wait();
   __shared__ double part[8];

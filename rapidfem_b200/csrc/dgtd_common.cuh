@@ -36,7 +36,17 @@ constexpr int kMaxOrder = 5;
 // stage loads its constant operands and allocates its TMEM meanwhile, on SMs the
 // previous stage has left: 12.4 -> 8.8 us per stage of 3,072 order-3 elements,
 // 8.3 -> 5.7 us of 384 order-2 elements, 81.3 -> 76.6 us of 82,944 order-3
-// elements.  (All stages of a run in one cooperative launch, synchronised tile by
+// elements.
+//
+// What earlier kernels of the stream write is not constant while such a kernel
+// runs, although nothing writes it after pdl_wait: it is read by plain loads
+// through pointers without __restrict__.  __ldg, and the non-coherent load that
+// const __restrict__ lets the compiler pick, ask for memory that no one writes
+// during the kernel, and a __restrict__ pointer's accesses need not stay below
+// the wait.  Both remain for what the host uploads: operator tables, element
+// records, index lists and weights.
+//
+// (All stages of a run in one cooperative launch, synchronised tile by
 // tile, measured 11.7, 5.8 and 77.1 us, and 1.14 times the time of single stages
 // at 663,552 order-4 elements.)
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

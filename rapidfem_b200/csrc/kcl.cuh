@@ -80,14 +80,27 @@ __device__ inline double kcl_factor(const KclCtl& c, double err_norm, double pre
   return reject ? fmax(f, c.shrink) : fmin(fmax(f, c.shrink), c.growth);
 }
 
-__global__ void k_kcl_begin(KclCtl* __restrict__ ctl, const float* __restrict__ y, float* __restrict__ ybak,
-                            int64_t n) {
+// dst = src over the grid's threads.  Four loads in flight per thread: the
+// pointers may alias as far as the compiler knows (pdl_wait says why), so it
+// would not move a load above the store before it.
+__device__ __forceinline__ void kcl_copy(float* dst, const float* src, int64_t n) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + 3 * step < n; i += 4 * step) {
+    const float a = src[i], b = src[i + step], c = src[i + 2 * step], d = src[i + 3 * step];
+    dst[i] = a;
+    dst[i + step] = b;
+    dst[i + 2 * step] = c;
+    dst[i + 3 * step] = d;
+  }
+  for (; i < n; i += step) dst[i] = src[i];
+}
+
+__global__ void k_kcl_begin(KclCtl* ctl, const float* y, float* ybak, int64_t n) {
   pdl_launch();
   pdl_wait();
   const bool run = ctl->status == kKclRunning && ctl->frame < ctl->steps;
-  if (run)
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-      ybak[i] = y[i];
+  if (run) kcl_copy(ybak, y, n);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctl->skip = run ? 0 : 1;
     if (run) ctl->h_try = fminf(ctl->h, ctl->dt - ctl->t_rel);
@@ -97,9 +110,8 @@ __global__ void k_kcl_begin(KclCtl* __restrict__ ctl, const float* __restrict__ 
 }
 
 // Block partials of the weighted squared embedded error (kcl.cl weighted_err_sq).
-__global__ void __launch_bounds__(256) k_kcl_err(const KclCtl* __restrict__ ctl, const float* __restrict__ y_old,
-                                                 const float* __restrict__ y_new, const float* __restrict__ err,
-                                                 double* __restrict__ partials, int64_t n) {
+__global__ void __launch_bounds__(256) k_kcl_err(const KclCtl* ctl, const float* y_old, const float* y_new,
+                                                 const float* err, double* partials, int64_t n) {
   pdl_launch();
   pdl_wait();
   if (ctl->skip) return;
@@ -123,8 +135,7 @@ __global__ void __launch_bounds__(256) k_kcl_err(const KclCtl* __restrict__ ctl,
 
 // err_norm = sqrt(sum / n), then the accept / reject decision of
 // gpu/operator.rs:848-887 and the frame bookkeeping.
-__global__ void __launch_bounds__(256) k_kcl_control(KclCtl* __restrict__ ctl, const double* __restrict__ partials,
-                                                     int nb, int64_t n) {
+__global__ void __launch_bounds__(256) k_kcl_control(KclCtl* ctl, const double* partials, int nb, int64_t n) {
   pdl_launch();
   pdl_wait();
   if (ctl->skip) return;
@@ -175,31 +186,26 @@ __global__ void __launch_bounds__(256) k_kcl_control(KclCtl* __restrict__ ctl, c
   }
 }
 
-__global__ void k_kcl_restore(const KclCtl* __restrict__ ctl, float* __restrict__ y, const float* __restrict__ ybak,
-                              int64_t n) {
+__global__ void k_kcl_restore(const KclCtl* ctl, float* y, const float* ybak, int64_t n) {
   pdl_launch();
   pdl_wait();
   if (ctl->skip || !ctl->restore) return;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = ybak[i];
+  kcl_copy(y, ybak, n);
 }
 
 // Frame record: the SoA state into row `record` of a device trajectory.
-__global__ void k_kcl_record_state(const KclCtl* __restrict__ ctl, const float* __restrict__ y,
-                                   float* __restrict__ traj, int64_t n) {
+__global__ void k_kcl_record_state(const KclCtl* ctl, const float* y, float* traj, int64_t n) {
   pdl_launch();
   pdl_wait();
   if (ctl->skip || ctl->record < 0) return;
-  float* row = traj + (int64_t)ctl->record * n;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    row[i] = y[i];
+  kcl_copy(traj + (int64_t)ctl->record * n, y, n);
 }
 
 // Frame record: linear functionals (one block each) into row `record`.
-__global__ void __launch_bounds__(256) k_kcl_record_fun(const KclCtl* __restrict__ ctl, const float* __restrict__ y,
+__global__ void __launch_bounds__(256) k_kcl_record_fun(const KclCtl* ctl, const float* y,
                                                         const int64_t* __restrict__ ptr,
                                                         const int64_t* __restrict__ idx,
-                                                        const double* __restrict__ w, double* __restrict__ out,
+                                                        const double* __restrict__ w, double* out,
                                                         int64_t n_fun) {
   pdl_launch();
   pdl_wait();

@@ -176,8 +176,8 @@ template <> struct KryVec<double> {
 // and w . w in the norm column.
 template <class B>
 __global__ void __launch_bounds__(kKrylovThreads, 2)
-k_kry_dots(const B* __restrict__ v0, const B* __restrict__ vb, int64_t len, int64_t n, int cols,
-           const B* __restrict__ w, double* __restrict__ partials, const int* skip) {
+k_kry_dots(const B* v0, const B* vb, int64_t len, int64_t n, int cols,
+           const B* w, double* partials, const int* skip) {
   pdl_launch();
   pdl_wait();
   if (*skip) return;
@@ -248,9 +248,8 @@ __device__ __forceinline__ void kry_proj(KrylovDev* st, const double* sums, int 
 // per SM) with the f32 update of an f32 basis.
 template <class B, int NC>
 __global__ void __launch_bounds__(kKrylovThreads, 2)
-k_kry_update_dots(KrylovDev* st, const B* __restrict__ v0, const B* __restrict__ vb, int64_t len, int64_t n,
-                  int j, B* __restrict__ w, const double* __restrict__ partials_in, int nb_in,
-                  double* __restrict__ partials_out, const int* skip) {
+k_kry_update_dots(KrylovDev* st, const B* v0, const B* vb, int64_t len, int64_t n,
+                  int j, B* w, const double* partials_in, int nb_in, double* partials_out, const int* skip) {
   pdl_launch();
   pdl_wait();
   static_assert(NC <= kKryCols, "columns");
@@ -318,9 +317,8 @@ k_kry_update_dots(KrylovDev* st, const B* __restrict__ v0, const B* __restrict__
 // second-pass update and the partial sums of |w|^2 (the norm column).
 template <class B, int NC>
 __global__ void __launch_bounds__(kKrylovThreads, 2)
-k_kry_update_norm(KrylovDev* st, const B* __restrict__ v0, const B* __restrict__ vb, int64_t len, int64_t n,
-                  int j, B* __restrict__ w, const double* __restrict__ partials_in, int nb_in,
-                  double* __restrict__ partials_out, const int* skip) {
+k_kry_update_norm(KrylovDev* st, const B* v0, const B* vb, int64_t len, int64_t n,
+                  int j, B* w, const double* partials_in, int nb_in, double* partials_out, const int* skip) {
   pdl_launch();
   pdl_wait();
   static_assert(NC <= kKryCols, "columns");
@@ -385,7 +383,7 @@ k_kry_update_norm(KrylovDev* st, const B* __restrict__ v0, const B* __restrict__
 // Partial sums of x^2 (slot 0 of each block's row).
 template <class B>
 __global__ void __launch_bounds__(kKrylovThreads, 2)
-k_kry_norm_partials(const B* __restrict__ x, int64_t n, double* __restrict__ partials) {
+k_kry_norm_partials(const B* x, int64_t n, double* partials) {
   pdl_launch();
   pdl_wait();
   __shared__ double red[kKrylovThreads / 32];
@@ -402,8 +400,7 @@ k_kry_norm_partials(const B* __restrict__ x, int64_t n, double* __restrict__ par
 // entries past n are written as the zero combination of zero entries).
 template <class B>
 __global__ void __launch_bounds__(kKrylovThreads, 2)
-k_kry_lincomb(const B* __restrict__ v0, const B* __restrict__ vb, int64_t len, int64_t n, const KrylovDev* st,
-              B* __restrict__ out) {
+k_kry_lincomb(const B* v0, const B* vb, int64_t len, int64_t n, const KrylovDev* st, B* out) {
   pdl_launch();
   pdl_wait();
   using KV = KryVec<B>;

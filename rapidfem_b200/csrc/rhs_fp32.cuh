@@ -117,9 +117,9 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
       if ((nfloat % C::PER16) == 0) {
         const V* s4 = reinterpret_cast<const V*>(src);
         V* d4 = reinterpret_cast<V*>(sY);
-        for (int i = tid; i < nfloat / C::PER16; i += blockDim.x) d4[i] = __ldg(s4 + i);
+        for (int i = tid; i < nfloat / C::PER16; i += blockDim.x) d4[i] = s4[i];
       } else {
-        for (int i = tid; i < nfloat; i += blockDim.x) sY[i] = __ldg(src + i);
+        for (int i = tid; i < nfloat; i += blockDim.x) sY[i] = src[i];
       }
     }
     {
@@ -168,8 +168,8 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
           qx = Z[3 * NP + vj]; qy = Z[4 * NP + vj]; qz = Z[5 * NP + vj];
         } else {
           const R* Z = P.y_in + (int64_t)nbr * 6 * NP;
-          px = __ldg(Z + 0 * NP + vj); py = __ldg(Z + 1 * NP + vj); pz = __ldg(Z + 2 * NP + vj);
-          qx = __ldg(Z + 3 * NP + vj); qy = __ldg(Z + 4 * NP + vj); qz = __ldg(Z + 5 * NP + vj);
+          px = Z[0 * NP + vj]; py = Z[1 * NP + vj]; pz = Z[2 * NP + vj];
+          qx = Z[3 * NP + vj]; qy = Z[4 * NP + vj]; qz = Z[5 * NP + vj];
         }
         jex = ex - px; jey = ey - py; jez = ez - pz;
         jhx = hx - qx; jhy = hy - qy; jhz = hz - qz;
@@ -312,7 +312,7 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
         for (int c = 0; c < 6; ++c) {
           const int64_t g = base + c * NP;
           R k = dy[c];
-          if (P.src_vec != nullptr) k = fma(P.src_g, __ldg(P.src_vec + g), k);
+          if (P.src_vec != nullptr) k = fma(P.src_g, P.src_vec[g], k);
           if (g == P.src_idx) k += P.src_g;
           R pv = (P.dt * M[43]) * k;
           if (P.read_p) pv = fma(P.a, P.p[g], pv);
@@ -343,7 +343,7 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
         for (int c = 0; c < 6; ++c) {
           const int64_t g = base + c * NP;
           R w = kry_sig * dy[c];
-          if (P.src_vec != nullptr) w = fma(kry_g, __ldg(P.src_vec + g), w);
+          if (P.src_vec != nullptr) w = fma(kry_g, P.src_vec[g], w);
           if (g == P.src_idx) w += kry_g;
           P.out[g] = w;
         }
@@ -401,8 +401,8 @@ __device__ __forceinline__ void rhs_cc_flux(const RhsParamsT<R>& P, int64_t e0, 
         qx = Z[3 * NP + vj]; qy = Z[4 * NP + vj]; qz = Z[5 * NP + vj];
       } else {
         const R* Z = P.y_in + (int64_t)nbr * 6 * NP;
-        px = __ldg(Z + 0 * NP + vj); py = __ldg(Z + 1 * NP + vj); pz = __ldg(Z + 2 * NP + vj);
-        qx = __ldg(Z + 3 * NP + vj); qy = __ldg(Z + 4 * NP + vj); qz = __ldg(Z + 5 * NP + vj);
+        px = Z[0 * NP + vj]; py = Z[1 * NP + vj]; pz = Z[2 * NP + vj];
+        qx = Z[3 * NP + vj]; qy = Z[4 * NP + vj]; qz = Z[5 * NP + vj];
       }
       jex = ex - px; jey = ey - py; jez = ez - pz;
       jhx = hx - qx; jhy = hy - qy; jhz = hz - qz;
@@ -545,7 +545,7 @@ __device__ __forceinline__ void rhs_cc_pair_body(const RhsParamsT<R>& P, const O
       const V2* src = reinterpret_cast<const V2*>(P.y_in + e0 * 6 * NP);
       for (int i = tid; i < ne * (3 * NP); i += blockDim.x) {
         const int el = i / (3 * NP);
-        *reinterpret_cast<V2*>(sY + el * YS + 2 * (i - el * (3 * NP))) = __ldg(src + i);
+        *reinterpret_cast<V2*>(sY + el * YS + 2 * (i - el * (3 * NP))) = src[i];
       }
     }
     {
@@ -647,7 +647,7 @@ __device__ __forceinline__ void rhs_cc_pair_body(const RhsParamsT<R>& P, const O
               P.out[g] = dy;
             } else if (MODE == kModeLserk) {
               R k = dy;
-              if (P.src_vec != nullptr) k = fma(P.src_g, __ldg(P.src_vec + g), k);
+              if (P.src_vec != nullptr) k = fma(P.src_g, P.src_vec[g], k);
               if (g == P.src_idx) k += P.src_g;
               R pv = (P.dt * M[43]) * k;
               if (P.read_p) pv = fma(P.a, P.p[g], pv);
@@ -668,7 +668,7 @@ __device__ __forceinline__ void rhs_cc_pair_body(const RhsParamsT<R>& P, const O
               // Krylov matvec of a stored basis vector: its scale and the source
               // coefficient of the augmented system come from device memory
               R w = kry_sig * dy;
-              if (P.src_vec != nullptr) w = fma(kry_g, __ldg(P.src_vec + g), w);
+              if (P.src_vec != nullptr) w = fma(kry_g, P.src_vec[g], w);
               if (g == P.src_idx) w += kry_g;
               P.out[g] = w;
             }

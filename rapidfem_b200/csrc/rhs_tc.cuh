@@ -566,7 +566,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
 #pragma unroll
             for (int c = 0; c < 6; ++c)
 #pragma unroll
-              for (int i = 0; i < FN; ++i) tr[i][c] = __ldg(Z + gn[i] + c * NP);
+              for (int i = 0; i < FN; ++i) tr[i][c] = Z[gn[i] + c * NP];
           }
         } else if (kind == kPec) {
           // PEC ghost: [E] = 2 E_tan, [H] = 2 H_n (rhs.rs:1387-1402).  Both
@@ -762,7 +762,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
               for (int u = 0; u < 4; ++u) {
                 const int i = i0 + u;
                 if (lane_real && i < NP) {
-                  if (P.src_vec != nullptr) dy[u] = fmaf(P.src_g, __ldg(P.src_vec + g_row + i), dy[u]);
+                  if (P.src_vec != nullptr) dy[u] = fmaf(P.src_g, P.src_vec[g_row + i], dy[u]);
                   if (P.src_idx == g_row + i) dy[u] += P.src_g;
                 }
               }
@@ -795,7 +795,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
             for (int u = 0; u < 4; ++u) {
               float kk = dy[u];
               if (src_here && lane_real && i0 + u < NP) {
-                if (P.src_vec != nullptr) kk += __ldg(P.src_vec + g + u) * kcl_gs;
+                if (P.src_vec != nullptr) kk += P.src_vec[g + u] * kcl_gs;
                 if (P.src_idx == g + u) kk += kcl_gs;
               }
               const float fk = kcl_h * kk;
@@ -817,7 +817,7 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
                 for (int u = 0; u < 4; ++u) {
                   const int i = i0 + u;
                   if (lane_real && i < NP) {
-                    if (P.src_vec != nullptr) dy[u] = fmaf(kry_g, __ldg(P.src_vec + g_row + i), dy[u]);
+                    if (P.src_vec != nullptr) dy[u] = fmaf(kry_g, P.src_vec[g_row + i], dy[u]);
                     if (P.src_idx == g_row + i) dy[u] += kry_g;
                   }
                 }
