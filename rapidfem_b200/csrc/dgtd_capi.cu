@@ -34,6 +34,9 @@ namespace dgtd {
 static thread_local std::string g_last_error;
 int set_error(int code, const std::string& msg) {
   g_last_error = msg;
+  // A failed CUDA call also leaves its error for the next cudaGetLastError to
+  // find: taken out here, or the next launch, a good one, would report it.
+  if (code == DGTD_ERR_CUDA || code == DGTD_ERR_OOM || code == DGTD_ERR_NO_DEVICE) (void)cudaGetLastError();
   return code;
 }
 }  // namespace dgtd
