@@ -457,9 +457,14 @@ int dgtd_debug_tc_gemm(dgtd_ctx *ctx, const float *a, const float *b, float *c, 
  * DGTD_ERR_TIMEOUT through the same device flag a stage kernel raises, with
  * the time waited in *waited_s.  Nothing faults; the context stays usable. */
 int dgtd_debug_wait_timeout(dgtd_ctx *ctx, int64_t max_polls, double *waited_s);
-/* Per-phase cycle counters of the tensor-core RHS kernel (8 u64 in device
- * memory, accumulated by thread 0 of every CTA); recorded only by builds
- * compiled with -DDGTD_TC_PHASE_TIMERS, ignored otherwise.  NULL detaches. */
+/* Per-phase cycle counters of the tensor-core RHS kernel:
+ * DGTD_TC_PHASE_COUNTERS u64 in device memory, to which one thread of each role
+ * of every CTA adds its own (volume warps 0 waits, 1 work; flux warps 8 tile
+ * wait, 9 trace loads, 2 operand wait, 3 flux; epilogue 10 MMA wait, 4 slot
+ * waits, 5 work; control lane 6; copy lane 11 results wait, 7 store read).
+ * Recorded only by builds compiled with -DDGTD_TC_PHASE_TIMERS, ignored
+ * otherwise.  NULL detaches. */
+#define DGTD_TC_PHASE_COUNTERS 12
 int dgtd_debug_set_phase_clock(dgtd_op *op, void *d_counters);
 
 #ifdef __cplusplus

@@ -2671,10 +2671,10 @@ extern "C" int dgtd_debug_tc_gemm(dgtd_ctx* ctx, const float* a, const float* b,
   return DGTD_OK;
 }
 
-// Point the tensor-core kernel's phase counters (12 x u64, device memory) at
-// `d_counters`; only builds compiled with -DDGTD_TC_PHASE_TIMERS record them.
+// Point the tensor-core kernel's phase counters (device memory) at `d_counters`; only builds compiled with -DDGTD_TC_PHASE_TIMERS record them.
 extern "C" int dgtd_debug_set_phase_clock(dgtd_op* op, void* d_counters) {
   if (!op) return set_error(DGTD_ERR_BAD_ARG, "debug_set_phase_clock: null op");
+  static_assert(DGTD_TC_PHASE_COUNTERS == dgtd::kTcMarks, "the caller's buffer holds every counter");
   op->phase_clk = static_cast<unsigned long long*>(d_counters);
   return DGTD_OK;
 }

@@ -26,6 +26,15 @@ def test_library_exports_every_declared_symbol():
     assert len(_declared()) >= 30
 
 
+def test_phase_counter_buffer_holds_every_mark():
+    """The buffer size the header asks for covers each index the instrumented kernel adds to."""
+    header = open(os.path.join(ROOT, "include", "dgtd.h")).read()
+    kernel = open(os.path.join(ROOT, "rapidfem_b200", "csrc", "rhs_tc.cuh")).read()
+    want = int(re.search(r"#define DGTD_TC_PHASE_COUNTERS (\d+)", header).group(1))
+    assert want == int(re.search(r"kTcMarks = (\d+)", kernel).group(1))
+    assert want > max(int(i) for i in re.findall(r"DGTD_TC_MARK\((\d+)\)", kernel))
+
+
 def test_version_names_sm100a():
     from rapidfem_b200 import _native
     assert "sm_100a" in _native.version()
