@@ -1,6 +1,6 @@
-"""The tensor-core stage kernel's tile edges: the flux units (groups of four
-face nodes, whose last group is partly padding), every face kind in one tile,
-rough fields, tiles of which one element or all but one are real.
+"""The tensor-core stage kernel's tile edges: the flux units (groups of two face
+nodes, four at order 4, whose last group may be partly padding), every face kind
+in one tile, rough fields, tiles of which one element or all but one are real.
 
 Tolerance: a right-hand side is a sum of at most 3 Np + 4 Nfp (252) f32-class
 products; with random signs its relative error is about sqrt(252) 2^-24 times
