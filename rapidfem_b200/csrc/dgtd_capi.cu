@@ -1099,7 +1099,7 @@ extern "C" int dgtd_transient_probes(dgtd_op* op, const float* y0, float dt, int
   DGTD_TRY(dgtd_state_upload(op, y0));
   auto record = [&](int64_t row) -> int {
     if (n_probes == 0) return DGTD_OK;
-    CUDA_TRY(launch_pdl(k_gather_f32, (unsigned)grid_for(n_probes, 256, op->ctx->num_sms), 256, 0, op->stream(), 
+    CUDA_TRY(launch_pdl(k_gather_f32, (unsigned)grid_for(n_probes, 256, op->ctx->num_sms), 256, 0, op->stream(),
         op->y[op->cur].p, d_probe.p, n_probes, d_pv.p + row * n_probes));
     op->launches++;
     CUDA_TRY(cudaGetLastError());

@@ -29,14 +29,18 @@ constexpr int kMaxGather = 96;
 constexpr int kMaxOrder = 5;
 
 // Programmatic dependent launch: a kernel lets the next one in its stream be
-// placed as soon as all its own blocks run, and touches what earlier kernels
-// wrote (or will read) only after pdl_wait, which returns once they are complete
+// placed once all its own blocks have called pdl_launch (most kernels at once, a
+// tensor-core stage when it holds its TMEM, the layout conversions and the
+// CUDA-core stages at their end: their comments say why), and touches what earlier
+// kernels wrote (or will read) only after pdl_wait, which returns once they are complete
 // and their writes visible.  Every thread waits before anything else that can
 // end it, so a kernel never completes before its predecessors.  A tensor-core
 // stage loads its constant operands and allocates its TMEM meanwhile, on SMs the
 // previous stage has left: 12.4 -> 8.8 us per stage of 3,072 order-3 elements,
 // 8.3 -> 5.7 us of 384 order-2 elements, 81.3 -> 76.6 us of 82,944 order-3
-// elements.
+// elements.  (All stages of a run in one cooperative launch, synchronised tile by
+// tile, measured 11.7, 5.8 and 77.1 us, and 1.14 times the time of single stages
+// at 663,552 order-4 elements.)
 //
 // What earlier kernels of the stream write is not constant while such a kernel
 // runs, although nothing writes it after pdl_wait: it is read by plain loads
@@ -45,10 +49,6 @@ constexpr int kMaxOrder = 5;
 // during the kernel, and a __restrict__ pointer's accesses need not stay below
 // the wait.  Both remain for what the host uploads: operator tables, element
 // records, index lists and weights.
-//
-// (All stages of a run in one cooperative launch, synchronised tile by
-// tile, measured 11.7, 5.8 and 77.1 us, and 1.14 times the time of single stages
-// at 663,552 order-4 elements.)
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -8,7 +8,7 @@
 //   2. the numerical flux of all 4*Nfp face nodes of every element is formed
 //      (rhs.rs:1370-1441): the neighbour trace comes from shared memory when
 //      the neighbour is in the tile, else from L2/HBM;
-//   3. each thread owns one (element, node): 18 reference derivatives
+//   3. each thread owns one (element, node), at order 4 two: 18 reference derivatives
 //      D_k * F_c (rhs.rs:39-85), combined with J^-1 into curl H / -curl E;
 //   4. the LIFT sum over the 4*Nfp flux values (rhs.rs:1433-1439), the
 //      material scaling (rhs.rs:1443-1454), and the mode's epilogue:
@@ -25,14 +25,16 @@
 
 namespace dgtd {
 
+// One node per thread: every order but 4 (PairCfg, below).
 template <int N, class R = float, int TD = 1>
 struct Fp32Cfg {
+  static_assert(N != 4, "order 4 has two nodes per thread");
   static constexpr int NP = np_of(N);
   static constexpr int NFP = nfp_of(N);
   static constexpr int NF = 4 * NFP;
   // Elements per tile: ~256 threads (TD = 1) or half as many (TD = 2, the
   // small-tile engine), E even so the tile start stays 16B aligned.
-  static constexpr int E = (N == 1 ? 64 : N == 2 ? 24 : N == 3 ? 12 : N == 4 ? 8 : 4) / TD;
+  static constexpr int E = (N == 1 ? 64 : N == 2 ? 24 : N == 3 ? 12 : 4) / TD;
   static_assert(TD == 1 || TD == 2, "tile divisor");
   static constexpr int THREADS = ((E * NP + 31) / 32) * 32;
   static constexpr int TILE = E * 6 * NP;  // values of state per tile
@@ -202,7 +204,7 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
       if constexpr (N == 5 && sizeof(R) == 4) {
         // the element's state rows are 16-byte aligned (Np = 56): four nodes of
         // all six components per float4 (broadcast) load, same accumulation
-        // order (order 5: 14 % faster; orders 3 and 4 measured no gain)
+        // order (order 5: 14 % faster; order 3 measured no gain)
 #pragma unroll 2
         for (int j0 = 0; j0 < NP; j0 += 4) {
           float4 yv[6];
@@ -358,7 +360,8 @@ __device__ __forceinline__ void rhs_cc_body(const RhsParamsT<R>& P, const OpTabl
 // The numerical flux (rhs.rs:1370-1441) at the face nodes of a tile's `ne` elements
 // from e0 on, by all threads: states sY and fluxes sF with element strides YS, FS.
 // (As in rhs_cc_body, which keeps its own copy: called from there it cost order 5
-// 18 %.)
+// 18 %, and as long as order 5 needs the copy, calling it at the other orders
+// would spare no code.)
 template <int N, int YS, int FS, class R>
 __device__ __forceinline__ void rhs_cc_flux(const RhsParamsT<R>& P, int64_t e0, int ne, const R* sY, const R* sM,
                                             const uint8_t* sFn, const uint8_t* sG, R* sF) {
@@ -462,8 +465,8 @@ template <> struct Acc<double> {
 // (coalesced global accesses), and next to each other in the shared D and LIFT
 // rows: one vector load brings a row entry for both, a state or flux value is
 // read once for both, and f32 arithmetic is packed (f32x2).  48,000 elements:
-// 219 -> 173 us per f32 stage (TD = 2: 230 -> 180); f64, 10,368 elements: 1.26
-// times faster.  Not at the other orders, where the fluxes are the larger part and
+// 220 -> 172 us per f32 stage (TD = 2: 231 -> 178), 364 -> 311 us per f64 stage
+// (10,368 elements: 91 -> 64).  Not at the other orders, where the fluxes are the larger part and
 // half the threads form them: order 3 76 -> 75 us (1,296 elements: 9.2 -> 13.0),
 // order 2 59 -> 66, order 1 32 -> 43, order 5 193 -> 193 (f64: order 3 18.7 ->
 // 21.4 ms, order 5 23.7 -> 23.4, orders 1 and 2 the same).

@@ -43,9 +43,9 @@
 //
 // What bounds it: at order 4 the flux warps' chain of one tile (trace loads,
 // fluxes, operand stores), nearly as long as the tile period, with the
-// load/store pipe about 70 % busy; at order 3 that pipe, 86 % busy before the row
-// order below, a third of it replays of the face-node reads.  HBM and the tensor
-// pipe (18 to 24 %) are not.  One thread per (element, face, node group) with
+// load/store pipe 76 % busy; at order 3 that pipe, 84 % busy, half of the
+// shared-memory wavefronts replays (three quarters of them of loads).  HBM and
+// the tensor pipe (31 % busy at order 4, 19 % at order 3) are not.  One thread per (element, face, node group) with
 // vector operand stores, the loads of a face in neighbouring lanes, packed f32x2
 // arithmetic, a copy lane that refills a slot as soon as it is read and volume
 // warps of their own took five order-4 steps of the 48^3 box from 21.7 to 18.1
@@ -86,11 +86,7 @@
 
 namespace dgtd {
 
-constexpr int kTcTileE = 20;  // elements per tile at orders 1-4 (8 at order 5)
-// Warps by role: epilogue, 4 volume operand (both cover whole TMEM lane
-// quarters, quarter = warp % 4), then the order's flux warps, the control and
-// the copy warp.
-constexpr int kTcMarks = 12;  // phase timers
+constexpr int kTcMarks = 12;                 // phase timers (DGTD_TC_PHASE_COUNTERS)
 constexpr uint32_t kTcWaitLimit = 1u << 19;  // polls per bounded wait (about 2 s)
 
 __host__ __device__ constexpr int tc_r8(int x) { return (x + 7) & ~7; }
@@ -158,6 +154,9 @@ struct TcCfg {
   static constexpr int FG = (NFP + FN - 1) / FN;                                     // node groups per face
   static constexpr int UNITS_H = E * 2 * FG;                                   // units of a half
   static constexpr int WARPS_H = (UNITS_H + 31) / 32;                          // flux warps of a half
+  // Warps by role: epilogue, 4 volume operand (both cover whole TMEM lane
+  // quarters, quarter = warp % 4), then the order's flux warps, the control and
+  // the copy warp.
   static constexpr int EPI_WARPS = 12;
   static constexpr int VOL_WARP = EPI_WARPS, VOL_WARPS = 4, EPI_GROUPS = EPI_WARPS / 4;
   static constexpr int FLUX_WARP = VOL_WARP + VOL_WARPS;
@@ -408,7 +407,12 @@ rhs_tc_kernel(RhsParams P, TcTables T, int64_t n_tiles, int* err) {
   // whatever number of CTAs the compiler's register count lets an SM hold.
   pdl_launch();
   pdl_wait();
-  // a launch flagged off (adaptive stepping past its last attempt) has no tiles
+  // A launch flagged off (adaptive stepping past its last attempt, an Arnoldi step
+  // past convergence) has no tiles.  It has set itself up all the same: the flag
+  // belongs to an earlier kernel and is known only here.  In a queue of such
+  // launches the set-ups overlap: an exponential step of 3,072 order-3 elements
+  // with 9 of its 12 Arnoldi steps off takes 214 us, and took 340 us when each
+  // launch began after its predecessor's end and an off stage returned at once.
   const bool off = P.skip != nullptr && *P.skip;
   const int64_t n_my = !off && n_tiles > (int64_t)blockIdx.x
                            ? (n_tiles - (int64_t)blockIdx.x + gridDim.x - 1) / gridDim.x
