@@ -139,3 +139,34 @@ def test_order_4_pairs_at_tile_edges(ctx, n_tets):
         gop.set_engine(engine)
         assert rel_l2(gop.apply(y32), want) < 5e-6
     assert rel_l2(gop.apply_f64(y), orc.apply(y)) < 1e-11
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5])
+def test_wall_flux_of_a_nearly_normal_field(ctx, order):
+    """E at an oblique PEC wall, all but normal to it: the wall's flux is of the
+    tangential part (here 1e-3 of E) and has to be exact to the rounding of that
+    part, not of E.  The field is constant, so only walls have a flux, and the
+    difference of the upwind and the central right-hand side is its lifted
+    penalty alone (the volume terms are the same bits).  Against the FP32 engine,
+    which projects E first and reads the same records.
+
+    Tolerance: the 3xTF32 products leave 2^-21 of each LIFT term; a LIFT row's
+    terms cancel by a factor of up to about 10 over a face, so 5e-6.  Rounded as
+    E is, the flux is off by the order of 2^-24 / 1e-3 = 6e-5."""
+    box = O.structured_box(4, 4, 2)
+    side = sum(O.boundary_faces_on_plane(box, a, v) for a in (0, 1) for v in (0.0, 1.0)).any(axis=1)
+    wall = sum(O.boundary_faces_on_plane(box, 2, v) for v in (0.0, 1.0)).any(axis=1)
+    q, _ = np.linalg.qr(np.array([[2.0, 0.3, 0.5], [0.1, 1.5, 0.7], [0.4, 0.2, 1.0]]))
+    m = O.Mesh(np.ascontiguousarray(box.nodes @ q.T), box.tets)  # z walls: normal q[:, 2]
+    field = np.zeros(6)
+    field[:3] = q[:, 2] + 1e-3 * q[:, 0]
+    got = {}
+    for engine in (_native.ENGINE_TF32X3, _native.ENGINE_FP32):
+        dy = []
+        for alpha in (1.0, 0.0):
+            gop = G.GpuOperator(ctx, O.MaxwellOperator(m, order, alpha))
+            gop.set_engine(engine)
+            y = np.tile(field, gop.n_dof() // 6).astype(np.float32)
+            dy.append(gop.apply(y).astype(np.float64).reshape(m.n_tets, -1))
+        got[engine] = (dy[0] - dy[1])[wall & ~side]  # the side walls see E as tangential
+    assert rel_l2(got[_native.ENGINE_TF32X3], got[_native.ENGINE_FP32]) < 5e-6
